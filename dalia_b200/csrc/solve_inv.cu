@@ -254,12 +254,14 @@ __device__ __forceinline__ void strip_product(const double* M, int b, int c0, in
   }
 }
 
+// The rows that strip_product takes first: from rlo on, to the end of the
+// staged chunk that holds row rlo.
 __device__ __forceinline__ void preload_strip(const double* M, int b, int c0, int rlo, PreStrip& pre) {
   const int lane = threadIdx.x & 31, c = c0 + (lane & (PS_COLS - 1));
   pre.at = nullptr;
   if (c >= b) return;
   pre.at = M + c;
-  load_column(pre.at, b, rlo + 2 * (threadIdx.x >> 5) + (lane >> 4), min(b, PS_CHUNK), pre.m);
+  load_column(pre.at, b, rlo + 2 * (threadIdx.x >> 5) + (lane >> 4), min(b, (rlo / PS_CHUNK + 1) * PS_CHUNK), pre.m);
 }
 
 __global__ void __launch_bounds__(PS_THREADS) sweep_persist_kernel(const __grid_constant__ PSweep P) {
