@@ -15,8 +15,9 @@
 // in shared memory once per product, every result finished inside one CTA (a
 // row by one warp; a strip's column sums over all rows by one CTA, summed in
 // a fixed order, so results do not depend on scheduling), and each CTA asks
-// for the rows of its next product to be brought into L2 before it waits at
-// the barrier and loads the first part of it into registers.  A step, forward
+// for the rows of its next product (all of them, or of large products the
+// first few) to be brought into L2 before it waits at the barrier and loads
+// the first part of it into registers.  A step, forward
 // and backward: b = 300 9.7 and 17.3 -> 6.6 and 8.0 us, b = 1500 24.9 and 39.4
 // -> 11.5 and 13.5 us (2.3 and 2.0 TB/s), against four CTAs of 8 warps per SM
 // with partial column sums in global memory and none of the above.  The
@@ -39,6 +40,8 @@ constexpr int PS_WARPS = PS_THREADS / 32;
 constexpr int PS_MAXI = 64;
 constexpr int PS_COLS = 16;    // columns of a backward strip (a 128-byte segment per row)
 constexpr int PS_CHUNK = 4096;  // vector entries staged at a time
+constexpr double PS_BIG_BYTES = 64e6;         // of the larger product of a step: half of L2
+constexpr int PS_BIG_FETCH = (12 << 20) / 8;  // entries asked for ahead of a barrier when it is larger
 constexpr long long PS_SPIN_LIMIT = 1LL << 24;
 
 struct PInst {
@@ -48,13 +51,14 @@ struct PInst {
   double* x;         // n b + a, in place
   double* t;         // b: right-hand side of a step's second product
   int n, b, a, vlo;
-  int row0;          // first row of this instance in the batch
+  int row0, pair0;   // first row, and first pair of rows, of this instance in the batch
   int strip0;        // first strip of this instance in the batch
 };
 
 struct PSweep {
   int count, trans, s0, s1;
   int units;      // rows (forward) or strips (backward) of all instances
+  int pairs;      // pairs of rows of all instances
   unsigned* bar;  // arrivals
   int* abort_flag;
   PInst inst[PS_MAXI];
@@ -157,26 +161,37 @@ __device__ __forceinline__ double warp_dot(const double* M, const double* sv, in
   return s;
 }
 
+// Rows of a CTA that are not contiguous: those numbered mid and up lie skip
+// rows further down.
+struct Gap {
+  int mid, skip;
+};
+template <bool GAP>
+__device__ __forceinline__ int row_of(int q, Gap gap) {
+  return GAP && q >= gap.mid ? q + gap.skip : q;
+}
+
 // out[r] = (in ? in[r] : 0) + sign sum_{k < len(r)} M[r][k] v[k] for rows
 // [r0, r1), len(r) = r + 1 for a lower-triangular M, else b.
+template <bool GAP = false>
 __device__ __forceinline__ void rows_product(const double* M, int b, int r0, int r1, bool tri, const double* v,
                                              const double* in, double sign, double* out, double* sv,
-                                             const PreRow& pre) {
+                                             const PreRow& pre, Gap gap = Gap()) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const bool once = b <= PS_CHUNK;  // the whole vector stays staged
   __syncthreads();                  // the previous product's reads of sv
   if (once) {
-    stage(sv, v, tri ? r1 : b);
+    stage(sv, v, tri ? row_of<GAP>(r1 - 1, gap) + 1 : b);
     __syncthreads();
   }
   for (int rb = r0; rb < r1; rb += PS_WARPS) {
-    const int r = rb + warp;
-    const int len = r < r1 ? (tri ? r + 1 : b) : 0;
+    const int q = rb + warp, r = row_of<GAP>(q, gap);
+    const int len = q < r1 ? (tri ? r + 1 : b) : 0;
     double s = 0.0;
     if (once) {
       s = warp_dot(M + (size_t)r * b, sv, len, lane, pre);
     } else {
-      const int top = tri ? min(r1, rb + PS_WARPS) : b;
+      const int top = tri ? row_of<GAP>(min(r1, rb + PS_WARPS) - 1, gap) + 1 : b;
       for (int k0 = 0; k0 < top; k0 += PS_CHUNK) {
         __syncthreads();
         stage(sv, v + k0, min(PS_CHUNK, top - k0));
@@ -185,14 +200,16 @@ __device__ __forceinline__ void rows_product(const double* M, int b, int r0, int
         s += warp_dot(M + (size_t)r * b + k0, sv, max(0, min(PS_CHUNK, len - k0)), lane, PreRow());
       }
     }
-    if (lane == 0 && r < r1) out[r] = (in ? __ldcg(in + r) : 0.0) + sign * s;
+    if (lane == 0 && q < r1) out[r] = (in ? __ldcg(in + r) : 0.0) + sign * s;
   }
 }
 
-__device__ __forceinline__ void preload_row(const double* M, int b, int r0, int r1, bool tri, PreRow& pre) {
-  const int r = r0 + (threadIdx.x >> 5);
+template <bool GAP = false>
+__device__ __forceinline__ void preload_row(const double* M, int b, int r0, int r1, bool tri, PreRow& pre,
+                                            Gap gap = Gap()) {
+  const int q = r0 + (threadIdx.x >> 5), r = row_of<GAP>(q, gap);
   pre.at = nullptr;
-  if (b > PS_CHUNK || r >= r1) return;
+  if (b > PS_CHUNK || q >= r1) return;
   pre.at = M + (size_t)r * b;
   load_pairs(pre.at, tri ? r + 1 : b, threadIdx.x & 31, pre.m);
 }
@@ -264,6 +281,20 @@ __device__ __forceinline__ void preload_strip(const double* M, int b, int c0, in
   load_column(pre.at, b, rlo + 2 * (threadIdx.x >> 5) + (lane >> 4), min(b, (rlo / PS_CHUNK + 1) * PS_CHUNK), pre.m);
 }
 
+// BIG: a step's larger product has more than PS_BIG_BYTES.  Asking for all of
+// the next product then drives lines out of L2 before they are used, so a CTA
+// asks for PS_BIG_FETCH / grid entries ahead of a barrier only, about what
+// memory delivers during the barrier (8 to 32 MB measured alike).  Such steps
+// are bound by bandwidth, so the forward sweep's triangular product is split
+// by pairs of rows q and b - 1 - q: contiguous rows give the last CTA of a
+// block twice the average.  Forward and backward, all asked for against BIG:
+// 12 x 20 blocks of 1500 (216 MB) 2.14 and 2.28 -> 1.58 and 1.83 ms, 6 x 100
+// of 1500 (108 MB) 4.98 and 5.52 -> 4.06 and 4.82, 20 of 4000 (128 MB) 1.07 and
+// 1.22 -> 0.77 and 1.05.  Below the line all is better: 60 of 2500 (50 MB)
+// 1.52 and 2.06 against 1.38 and 2.11, 16 x 40 of 600 (46 MB) 1.32 and 1.42
+// against 1.34 and 1.46, 16 of 1117 (10 MB) 0.158 and 0.194 against 0.167 and
+// 0.198 ms.
+template <bool BIG>
 __global__ void __launch_bounds__(PS_THREADS) sweep_persist_kernel(const __grid_constant__ PSweep P) {
   __shared__ __align__(16) double sv[PS_CHUNK];
   __shared__ double red[PS_WARPS][PS_COLS];
@@ -276,6 +307,7 @@ __global__ void __launch_bounds__(PS_THREADS) sweep_persist_kernel(const __grid_
     for (int k = 0; k < P.count; ++k) {
       const PInst& I = P.inst[k];
       const int lo = P.trans == 0 ? I.row0 : I.strip0;
+      if (BIG && lo >= u1) break;
       const int cnt = P.trans == 0 ? I.b : (I.b + PS_COLS - 1) / PS_COLS;
       const int a = max(u0, lo), e = min(u1, lo + cnt);
       if (a < e) f(I, a - lo, e - lo);
@@ -291,24 +323,53 @@ __global__ void __launch_bounds__(PS_THREADS) sweep_persist_kernel(const __grid_
   const size_t fbb = (size_t)F.b * F.b;
   // lines of rows [r0, r1) of a b-wide block, or of 16-column strips [s0, s1)
   // of its rows from rlo on
+  const int room = PS_BIG_FETCH / (int)gridDim.x;
+  int left = room;
+  // m of the units of `per` entries each that may still be asked for
+  auto take = [&](int m, int per) {
+    if constexpr (BIG) {
+      m = min(m, left / per);
+      left -= m * per;
+    }
+    return m;
+  };
   auto fetch_rows = [&](const double* M, int b, int r0, int r1) {
-    const size_t e0 = (size_t)r0 * b, e1 = (size_t)r1 * b;
+    const size_t e0 = (size_t)r0 * b, e1 = (size_t)(r0 + take(r1 - r0, b)) * b;
     for (size_t e = e0 + 16 * threadIdx.x; e < e1; e += 16 * PS_THREADS) prefetch_l2(M + e);
   };
-  auto fetch_tri = [&](const double* M, int b, int r0, int r1) {
-    for (int r = r0 + (threadIdx.x >> 5); r < r1; r += PS_WARPS)
-      for (int k = 16 * (threadIdx.x & 31); k <= r; k += 512) prefetch_l2(M + (size_t)r * b + k);
+  auto fetch_tri = [&](const double* M, int b, int r0, int r1, Gap gap) {
+    const int e1 = r0 + take(r1 - r0, (b + 1) / 2);
+    for (int q = r0 + (threadIdx.x >> 5); q < e1; q += PS_WARPS)
+      for (int r = row_of<BIG>(q, gap), k = 16 * (threadIdx.x & 31); k <= r; k += 512)
+        prefetch_l2(M + (size_t)r * b + k);
   };
   auto fetch_strips = [&](const double* M, int b, int s0, int s1, bool tri) {
-    const int w = s1 - s0, rlo = tri ? PS_COLS * s0 : 0;
+    const int rlo = tri ? PS_COLS * s0 : 0, w = take(s1 - s0, PS_COLS * (b - rlo));
     for (int q = threadIdx.x; q < (b - rlo) * w; q += PS_THREADS)
       prefetch_l2(M + (size_t)(rlo + q / w) * b + PS_COLS * (s0 + q % w));
+  };
+  // f(instance, first, last, gap): this CTA's rows of the forward sweep's
+  // triangular products; BIG: pairs [a, e) of an instance, which are its rows
+  // [a, e) and [b - e, b - a) (the middle row of an odd b once)
+  auto each_tri = [&](auto f) {
+    if constexpr (BIG) {
+      const int q0 = (int)((long long)P.pairs * blockIdx.x / gridDim.x);
+      const int q1 = (int)((long long)P.pairs * (blockIdx.x + 1) / gridDim.x);
+      for (int k = 0; k < P.count && P.inst[k].pair0 < q1; ++k) {
+        const PInst& I = P.inst[k];
+        const int a = max(q0 - I.pair0, 0), e = min(q1 - I.pair0, (I.b + 1) / 2), hi = max(I.b - e, e);
+        if (a < e) f(I, a, e + I.b - a - hi, Gap{e, hi - e});
+      }
+    } else {
+      each([&](const PInst& I, int r0, int r1) { f(I, r0, r1, Gap()); });
+    }
   };
 
   if (P.trans == 0) {
     PreRow pre;
     if (P.s0 > 0 && P.s0 < F.n) preload_row(F.L + (P.s0 - 1) * fbb, F.b, f0, f1, false, pre);
     for (int st = P.s0; st < P.s1; ++st) {
+      left = room;
       each([&](const PInst& I, int r0, int r1) {
         if (st >= I.n) return;
         double* xi = I.x + (size_t)st * I.b;
@@ -318,18 +379,34 @@ __global__ void __launch_bounds__(PS_THREADS) sweep_persist_kernel(const __grid_
         } else {
           for (int r = r0 + threadIdx.x; r < r1; r += PS_THREADS) I.t[r] = __ldcg(xi + r);
         }
-        fetch_tri(I.V + (size_t)(st - I.vlo) * I.b * I.b, I.b, r0, r1);
+        if constexpr (!BIG) fetch_tri(I.V + (size_t)(st - I.vlo) * I.b * I.b, I.b, r0, r1, Gap());
       });
       pre.at = nullptr;
-      if (st < F.n) preload_row(F.V + (st - F.vlo) * fbb, F.b, f0, f1, true, pre);
+      if constexpr (BIG) {
+        bool first = true;
+        each_tri([&](const PInst& I, int r0, int r1, Gap gap) {
+          const double* Vi = I.V + (size_t)(st - I.vlo) * I.b * I.b;
+          if (st < I.n) fetch_tri(Vi, I.b, r0, r1, gap);
+          if (st < I.n && first) preload_row<true>(Vi, I.b, r0, r1, true, pre, gap);
+          first = false;
+        });
+      } else if (st < F.n) {
+        preload_row(F.V + (st - F.vlo) * fbb, F.b, f0, f1, true, pre);
+      }
       if (!grid_barrier(P, gen)) return;
-      each([&](const PInst& I, int r0, int r1) {
+      left = room;
+      each_tri([&](const PInst& I, int r0, int r1, Gap gap) {
         if (st >= I.n) return;
         // y_i = V_i t
-        rows_product(I.V + (size_t)(st - I.vlo) * I.b * I.b, I.b, r0, r1, true, I.t, nullptr, 1.0,
-                     I.x + (size_t)st * I.b, sv, pre);
-        if (st + 1 < min(P.s1, I.n)) fetch_rows(I.L + (size_t)st * I.b * I.b, I.b, r0, r1);
+        rows_product<BIG>(I.V + (size_t)(st - I.vlo) * I.b * I.b, I.b, r0, r1, true, I.t, nullptr, 1.0,
+                          I.x + (size_t)st * I.b, sv, pre, gap);
+        if constexpr (!BIG)
+          if (st + 1 < min(P.s1, I.n)) fetch_rows(I.L + (size_t)st * I.b * I.b, I.b, r0, r1);
       });
+      if constexpr (BIG)
+        each([&](const PInst& I, int r0, int r1) {
+          if (st + 1 < min(P.s1, I.n)) fetch_rows(I.L + (size_t)st * I.b * I.b, I.b, r0, r1);
+        });
       pre.at = nullptr;
       if (st + 1 < min(P.s1, F.n)) preload_row(F.L + st * fbb, F.b, f0, f1, false, pre);
       if (!grid_barrier(P, gen)) return;
@@ -345,6 +422,7 @@ __global__ void __launch_bounds__(PS_THREADS) sweep_persist_kernel(const __grid_
   }
   for (int st = P.s0; st < P.s1; ++st) {
     const int fi = F.n - 1 - st;  // the first instance's block
+    left = room;
     each([&](const PInst& I, int s0, int s1) {
       const int i = I.n - 1 - st;
       if (i < 0) return;
@@ -366,6 +444,7 @@ __global__ void __launch_bounds__(PS_THREADS) sweep_persist_kernel(const __grid_
     pre.at = nullptr;
     if (fi >= 0) preload_strip(F.V + (fi - F.vlo) * fbb, F.b, PS_COLS * f0, PS_COLS * f0, pre);
     if (!grid_barrier(P, gen)) return;
+    left = room;
     each([&](const PInst& I, int s0, int s1) {
       const int i = I.n - 1 - st;
       if (i < 0) return;
@@ -412,6 +491,7 @@ int sweep_inv_steps(int count, const int* n, const int* b, const int* a, const d
   P.s1 = s1;
   P.abort_flag = abort_flag;
   size_t off = 0;
+  double bytes = 0;  // of the step's larger product
   for (int k = 0; k < count; ++k) {
     PInst& I = P.inst[k];
     I.L = n[k] > 1 ? L[k] : nullptr;
@@ -426,13 +506,17 @@ int sweep_inv_steps(int count, const int* n, const int* b, const int* a, const d
     off += sweep_inv_work(n[k], b[k], a[k]);
     if (trans == 0) I.row0 = P.units;
     else I.strip0 = P.units;
+    I.pair0 = P.pairs;
+    P.pairs += (b[k] + 1) / 2;
+    bytes += 8.0 * b[k] * b[k];
     P.units += trans == 0 ? b[k] : (b[k] + PS_COLS - 1) / PS_COLS;
   }
   // barrier words after the instances' scratch
   P.bar = reinterpret_cast<unsigned*>(work + off);
   if (cudaMemsetAsync(P.bar, 0, 2 * sizeof(unsigned), s) != cudaSuccess) return cudaErrorUnknown;
+  auto kernel = bytes > PS_BIG_BYTES ? sweep_persist_kernel<true> : sweep_persist_kernel<false>;
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, sweep_persist_kernel, PS_THREADS, 0) != cudaSuccess ||
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, PS_THREADS, 0) != cudaSuccess ||
       occ <= 0)
     return cudaErrorUnknown;
   const int sms = device_sm_count();
@@ -441,7 +525,7 @@ int sweep_inv_steps(int count, const int* n, const int* b, const int* a, const d
   const int grid = std::min(most, cand == 0 ? sms : cand == 1 ? std::max(1, sms / 2) : std::min(occ, 2) * sms);
   void* args[] = {&P};
   bta::ProfScope _ps(bta::PROF_SWEEP, s);
-  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(sweep_persist_kernel), dim3(grid),
+  return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(grid),
                                      dim3(PS_THREADS), args, 0, s);
 }
 

@@ -1,7 +1,8 @@
-"""The backward sweep through block inverses for blocks wider than the 4096
-vector entries that are staged at a time: strips from column 4096 on that are
+"""Sweeps through block inverses with large products: blocks wider than the 4096
+vector entries that are staged at a time, whose strips from column 4096 on are
 the first of a CTA's share (from b = 4113 on with one CTA per SM), alone and
-beside a smaller instance."""
+beside a smaller instance; and steps of more than 64 MB, whose rows are dealt
+in pairs."""
 import numpy as np
 import pytest
 
@@ -14,6 +15,14 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("sizes", [[(2, 4500, 3)], [(1, 5025, 0)], [(2, 4500, 0), (2, 4500, 1)],
                                    [(3, 130, 0), (2, 4500, 3)], [(1, 8210, 2)]])
 def test_wide_blocks_solve_with_the_factor(sizes, cand, monkeypatch):
+    base.test_sweeps_solve_with_the_factor(sizes, cand, monkeypatch)
+
+
+# a step's larger product has more than 64 MB: rows in pairs, odd and even b, an instance of few rows among them
+@pytest.mark.parametrize("cand", range(2))
+@pytest.mark.parametrize("sizes", [[(2, 2900, 3)], [(2, 1999, 2), (1, 65, 1), (3, 2500, 0)], [(1, 4095, 0)],
+                                   [(2, 517, 1)] * 33])
+def test_large_products_solve_with_the_factor(sizes, cand, monkeypatch):
     base.test_sweeps_solve_with_the_factor(sizes, cand, monkeypatch)
 
 
