@@ -32,9 +32,12 @@ struct TrtriDev {
 };
 
 constexpr int TRTRI_MAXI = 64;
+constexpr double COLUMN_WORK = 0.72;  // block_trtri
 
 struct TrtriBatch {
   int count, total;
+  int zeros;     // tasks of diagonal tiles clear the column above
+  int nqmax;     // largest nq
   int* flags;    // tile (p, c) of a block written
   int* counter;  // next task
   int* abort_flag;
@@ -62,10 +65,12 @@ __device__ __forceinline__ void trtri_load(double* As, double* Bs, const double*
 // acc += A[:, k0:kend] B[k0:kend, :] with A = rows x (.) at Arow, B = (.) x cols
 // at Bcol (both row stride ld), through a cp.async ring; the 64 rows of B
 // from row 64 k on are read once gate[k] is set.  Returns false when a wait
-// gave up.  VEC: every row is 16-byte aligned.
+// gave up.  VEC: every row is 16-byte aligned.  own: all rows of B are there (a
+// run-time value also where it is always true: the loop compiled without its
+// test of the gates took 3 to 6 % longer).
 template <bool VEC>
 __device__ __forceinline__ bool trtri_stream(const double* Arow, int rows, const double* Bcol, int cols, int k0,
-                                             int kend, int ld, const int* gate, int* abort_flag, int* s_flag,
+                                             int kend, int ld, bool own, const int* gate, int* abort_flag, int* s_flag,
                                              double* smem, double (&acc)[2][4][4], int tid, int wm, int wn, int g,
                                              int t) {
   double* As = smem;
@@ -74,14 +79,14 @@ __device__ __forceinline__ bool trtri_stream(const double* Arow, int rows, const
   const int nslab = (kend - k0) / TK;
   // the leading rows already written: one scan of their flags (relaxed loads
   // in flight together, one fence), later ones are waited for one by one
-  if (tid == 0) {
+  if (tid == 0 && !own) {
     int k = k0 / T;
     while (k < kend / T && ld_relaxed(gate + k) >= 1) ++k;
     __threadfence();
     s_flag[1] = k * T;
   }
   __syncthreads();
-  const int ready = s_flag[1];
+  const int ready = own ? kend : s_flag[1];
   bool ok = true;
   auto issue = [&](int j) {
     const int k = k0 + j * TK;
@@ -130,16 +135,18 @@ __device__ __forceinline__ bool trtri_stream(const double* Arow, int rows, const
 
 // Inverses of lower-triangular blocks, tile by tile:
 //   X(c, c) = Linv_cc,  X(p, c) = -Linv_pp sum_{k=c}^{p-1} L(p, k) X(k, c)   (p > c).
+// The sums are bound by the FP64 tensor pipe.
 // One task per tile, claimed by distance p - c from the diagonal (all blocks
 // of all instances of a distance before the next one), so a task waits only
-// on earlier tasks; it streams its sum as the tiles above it become final.
-// The sums are bound by the FP64 tensor pipe.  One task per tile, not one
-// CTA per tile column: a column is a serial chain of up to nq^2 / 2 tile
-// products, which for few blocks outlasts everything else (16 blocks of 1117:
-// 1.66 ms, odd rows loaded one element at a time; now 0.42 ms), and one
-// launch for all instances fills the GPU (12 x 20 blocks of 1500: 19.1 -> 11.7 ms,
-// 23 TF/s).
-// A task at distance 0 inverts the diagonal tile and clears its column above.
+// on earlier tasks; it streams its sum as the tiles above it become final.  A
+// task at distance 0 inverts the diagonal tile and clears its column above.
+// Many blocks are done with a CTA per tile column instead, the longest first,
+// after a launch for the diagonal tiles: no flags and no waits (tasks lose 7 %
+// to them), but a serial chain of up to nq^2 / 2 tile products, which for few
+// blocks outlasts everything else (16 blocks of 1117: 0.81 ms, by tiles 0.43).
+// The columns are not claimed by resident CTAs: the SMs take a long, a middle
+// and a short one each from the launch's order (claimed: 2 to 5 % slower).
+template <bool COL>
 __global__ void __launch_bounds__(THREADS, 3) block_trtri_kernel(const __grid_constant__ TrtriBatch B) {
   extern __shared__ __align__(16) double sm[];
   double* As = sm;
@@ -148,25 +155,27 @@ __global__ void __launch_bounds__(THREADS, 3) block_trtri_kernel(const __grid_co
   __shared__ int s_task[4], s_flag[2];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int wm = warp >> 1, wn = warp & 1, g = lane >> 2, t = lane & 3;
-  int dist = 0, before = 0;  // thread 0: tasks of distances < dist
+  int dist = COL ? 1 : 0, before = 0;  // thread 0: tasks of distances < dist
   for (;;) {
     __syncthreads();
     if (tid == 0) {
-      const int ti = atomicAdd(B.counter, 1);
+      const int ti = COL ? (int)blockIdx.x : atomicAdd(B.counter, 1);
       s_task[0] = -1;
       while (ti < B.total) {
+        const int len = B.nqmax - dist;  // COL: columns of len tiles below the diagonal one, the longest first
         int local = ti - before, cnt = 0, k = 0;
         for (; k < B.count; ++k) {
-          const int m = B.inst[k].n * max(0, B.inst[k].nq - dist);
+          const int nq = B.inst[k].nq;
+          const int m = B.inst[k].n * (COL ? (nq > len ? 1 : 0) : max(0, nq - dist));
           if (local < m) break;
           local -= m;
           cnt += m;
         }
         if (k < B.count) {
-          const int w = B.inst[k].nq - dist;
+          const int nq = B.inst[k].nq, w = COL ? 1 : nq - dist;
           s_task[0] = k;
           s_task[1] = local / w;
-          s_task[2] = local % w;
+          s_task[2] = COL ? nq - 1 - len : local % w;
           s_task[3] = dist;
           break;
         }
@@ -177,20 +186,16 @@ __global__ void __launch_bounds__(THREADS, 3) block_trtri_kernel(const __grid_co
     __syncthreads();
     if (s_task[0] < 0) break;
     const TrtriDev& I = B.inst[s_task[0]];
-    const int i = s_task[1], c = s_task[2], p = c + s_task[3];
+    const int i = s_task[1], c = s_task[2];
     const int b = I.b, nq = I.nq;
     const double* Di = I.D + (size_t)i * b * b;
     double* Oi = I.out + (size_t)i * b * b;
     int* gate = B.flags + I.flag0 + ((size_t)i * nq + c) * nq;
-    const int wc = min(T, b - c * T), rp = min(T, b - p * T);
-    double* o = Oi + (size_t)(p * T) * b + c * T;
+    const int wc = min(T, b - c * T);
     const bool vec = ((b & 1) == 0) &&
                      (((reinterpret_cast<uintptr_t>(Di) | reinterpret_cast<uintptr_t>(Oi)) & 15) == 0);
-    if (p == c) {
-      if (vec) load_async<SG>(As, Di + (size_t)(c * T) * b + c * T, b, wc, wc, tid);
-      else load<SG>(As, Di + (size_t)(c * T) * b + c * T, b, wc, wc, tid);
-      cp_async_commit();
-      // zeros above the diagonal tile
+    // above the diagonal tile
+    auto zeros = [&]() {
       for (int idx = 2 * tid; idx < c * T * T; idx += 2 * THREADS) {
         double* z = Oi + (size_t)(idx >> 6) * b + c * T + (idx & 63);
         if (vec && (idx & 63) + 1 < wc) {
@@ -200,6 +205,13 @@ __global__ void __launch_bounds__(THREADS, 3) block_trtri_kernel(const __grid_co
           if ((idx & 63) + 1 < wc) z[1] = 0.0;
         }
       }
+    };
+    if (s_task[3] == 0) {  // never with COL
+      double* o = Oi + (size_t)(c * T) * b + c * T;
+      if (vec) load_async<SG>(As, Di + (size_t)(c * T) * b + c * T, b, wc, wc, tid);
+      else load<SG>(As, Di + (size_t)(c * T) * b + c * T, b, wc, wc, tid);
+      cp_async_commit();
+      if (B.zeros) zeros();
       cp_async_wait<0>();
       __syncthreads();
       for (int r = wc + tid; r < T; r += THREADS) As[r * SG + r] = 1.0;
@@ -213,87 +225,102 @@ __global__ void __launch_bounds__(THREADS, 3) block_trtri_kernel(const __grid_co
       if (tid == 0) st_release(gate + c, 1);
       continue;
     }
-    double acc[2][4][4];
-    zero_acc(acc);
-    const double* Arow = Di + (size_t)(p * T) * b;
-    // Linv_pp (a task of distance 0 wrote it) is fetched during the sum when
-    // it is there already
-    const double* Lpp = Oi + (size_t)(p * T) * b + p * T;
-    const int* pgate = B.flags + I.flag0 + ((size_t)i * nq + p) * nq + p;
-    if (tid == 0) s_flag[0] = ld_acquire(pgate) >= 1;
-    __syncthreads();
-    const bool fetched = s_flag[0] != 0;
-    auto fetch = [&]() {
-      if (vec) load_async<SG>(Ys, Lpp, b, rp, rp, tid);
-      else load_shifted_async<T, T, SG>(Ys, Lpp, b, rp, 0, rp, tid);
-      cp_async_commit();
-    };
-    if (fetched) fetch();
-    if (!(vec ? trtri_stream<true>(Arow, rp, Oi + c * T, wc, c * T, p * T, b, gate, B.abort_flag, s_flag, As, acc, tid,
-                                   wm, wn, g, t)
-              : trtri_stream<false>(Arow, rp, Oi + c * T, wc, c * T, p * T, b, gate, B.abort_flag, s_flag, As, acc,
-                                    tid, wm, wn, g, t)))
-      continue;
-    if (!fetched) {
-      if (tid == 0) s_flag[0] = wait_ge(pgate, 1, B.abort_flag) ? 1 : 0;
+    // a tile, or the tiles of a column one after the other: those are read back
+    // by this CTA alone (a barrier orders them)
+    const bool own = COL && !B.zeros;  // COL: always
+    int p = COL ? c + 1 : c + s_task[3];
+    const int pend = COL ? nq : p + 1;
+    if (COL) {
+      zeros();
+    }
+    for (; p < pend; ++p) {
+      const int rp = min(T, b - p * T);
+      double* o = Oi + (size_t)(p * T) * b + c * T;
+      double acc[2][4][4];
+      zero_acc(acc);
+      const double* Arow = Di + (size_t)(p * T) * b;
+      // Linv_pp (a task of distance 0 wrote it) is fetched during the sum when
+      // it is there already (for a column it always is)
+      const double* Lpp = Oi + (size_t)(p * T) * b + p * T;
+      const int* pgate = B.flags + I.flag0 + ((size_t)i * nq + p) * nq + p;
+      if (!COL) {
+        if (tid == 0) s_flag[0] = ld_acquire(pgate) >= 1;
+        __syncthreads();
+      }
+      const bool fetched = COL || s_flag[0] != 0;
+      auto fetch = [&]() {
+        if (vec) load_async<SG>(Ys, Lpp, b, rp, rp, tid);
+        else load_shifted_async<T, T, SG>(Ys, Lpp, b, rp, 0, rp, tid);
+        cp_async_commit();
+      };
+      if (fetched) fetch();
+      if (!(vec ? trtri_stream<true>(Arow, rp, Oi + c * T, wc, c * T, p * T, b, own, gate, B.abort_flag, s_flag, As,
+                                          acc, tid, wm, wn, g, t)
+                : trtri_stream<false>(Arow, rp, Oi + c * T, wc, c * T, p * T, b, own, gate, B.abort_flag, s_flag, As,
+                                           acc, tid, wm, wn, g, t)))
+        break;
+      if (!fetched) {
+        if (tid == 0) s_flag[0] = wait_ge(pgate, 1, B.abort_flag) ? 1 : 0;
+        __syncthreads();
+        if (!s_flag[0]) break;
+        fetch();
+      }
+      // As[n][j] = acc[j][n] (the slab ring is free again)
+#pragma unroll
+      for (int mi = 0; mi < 2; ++mi)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int j = wm * 32 + mi * 16 + g + h * 8;
+#pragma unroll
+          for (int ni = 0; ni < 4; ++ni)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) As[(wn * 32 + ni * 8 + 2 * t + e) * SG + j] = acc[mi][ni][h * 2 + e];
+        }
+      cp_async_wait<0>();
       __syncthreads();
-      if (!s_flag[0]) continue;
-      fetch();
-    }
-    // As[n][j] = acc[j][n] (the slab ring is free again)
+      // X = -Linv_pp acc: Linv_pp is lower triangular (row tile mi sums k < 16 (mi + 1));
+      // a warp owns 16 whole columns, so the four have the same work
+      const int shl = vec ? 0 : row_parity(Lpp, b, g);
+      double x[4][2][4];
 #pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
+      for (int mi = 0; mi < 4; ++mi)
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int j = wm * 32 + mi * 16 + g + h * 8;
+        for (int ni = 0; ni < 2; ++ni)
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
+          for (int e = 0; e < 4; ++e) x[mi][ni][e] = 0.0;
 #pragma unroll
-          for (int e = 0; e < 2; ++e) As[(wn * 32 + ni * 8 + 2 * t + e) * SG + j] = acc[mi][ni][h * 2 + e];
-      }
-    cp_async_wait<0>();
-    __syncthreads();
-    // X = -Linv_pp acc: Linv_pp is lower triangular (row tile mi sums k < 16 (mi + 1));
-    // a warp owns 16 whole columns, so the four have the same work
-    const int shl = vec ? 0 : row_parity(Lpp, b, g);
-    double x[4][2][4];
+      for (int kk = 0; kk < T; kk += 4) {
+        const double b0 = As[(16 * warp + g) * SG + kk + t], b1 = As[(16 * warp + 8 + g) * SG + kk + t];
 #pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-      for (int ni = 0; ni < 2; ++ni)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) x[mi][ni][e] = 0.0;
-#pragma unroll
-    for (int kk = 0; kk < T; kk += 4) {
-      const double b0 = As[(16 * warp + g) * SG + kk + t], b1 = As[(16 * warp + 8 + g) * SG + kk + t];
-#pragma unroll
-      for (int mi = kk / 16; mi < 4; ++mi) {
-        const double* l = Ys + (16 * mi + g) * SG + kk + t + shl;
-        const double a0 = l[0], a1 = l[8 * SG];
-        dmma16x8x4(x[mi][0], a0, a1, b0);
-        dmma16x8x4(x[mi][1], a0, a1, b1);
-      }
-    }
-#pragma unroll
-    for (int mi = 0; mi < 4; ++mi)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int r = 16 * mi + g + h * 8;
-        if (r >= rp) continue;
-#pragma unroll
-        for (int ni = 0; ni < 2; ++ni) {
-          const int n = 16 * warp + ni * 8 + 2 * t;
-          double* dst = o + (size_t)r * b + n;
-          if (vec && n + 1 < wc) {
-            *reinterpret_cast<double2*>(dst) = make_double2(-x[mi][ni][h * 2], -x[mi][ni][h * 2 + 1]);
-          } else {
-            if (n < wc) dst[0] = -x[mi][ni][h * 2];
-            if (n + 1 < wc) dst[1] = -x[mi][ni][h * 2 + 1];
-          }
+        for (int mi = kk / 16; mi < 4; ++mi) {
+          const double* l = Ys + (16 * mi + g) * SG + kk + t + shl;
+          const double a0 = l[0], a1 = l[8 * SG];
+          dmma16x8x4(x[mi][0], a0, a1, b0);
+          dmma16x8x4(x[mi][1], a0, a1, b1);
         }
       }
-    __syncthreads();
-    if (tid == 0) st_release(gate + p, 1);
+#pragma unroll
+      for (int mi = 0; mi < 4; ++mi)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int r = 16 * mi + g + h * 8;
+          if (r >= rp) continue;
+#pragma unroll
+          for (int ni = 0; ni < 2; ++ni) {
+            const int n = 16 * warp + ni * 8 + 2 * t;
+            double* dst = o + (size_t)r * b + n;
+            if (vec && n + 1 < wc) {
+              *reinterpret_cast<double2*>(dst) = make_double2(-x[mi][ni][h * 2], -x[mi][ni][h * 2 + 1]);
+            } else {
+              if (n < wc) dst[0] = -x[mi][ni][h * 2];
+              if (n + 1 < wc) dst[1] = -x[mi][ni][h * 2 + 1];
+            }
+          }
+        }
+      __syncthreads();
+      if (!COL && tid == 0) st_release(gate + p, 1);
+    }
+    if (COL) break;
   }
 }
 
@@ -336,17 +363,20 @@ size_t block_trtri_flags(int n, int b) {
 }
 
 int block_trtri(const TrtriInst* inst, int count, int* flags, int* abort_flag, cudaStream_t s) {
-  {
-    const int e = ensure_smem_attr(reinterpret_cast<const void*>(block_trtri_kernel), (int)TRTRI_SMEM);
+  for (const void* f : {reinterpret_cast<const void*>(block_trtri_kernel<false>),
+                        reinterpret_cast<const void*>(block_trtri_kernel<true>)}) {
+    const int e = ensure_smem_attr(f, (int)TRTRI_SMEM);
     if (e != cudaSuccess) return e;
   }
   int occ = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, block_trtri_kernel, THREADS, TRTRI_SMEM);
+  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, block_trtri_kernel<false>, THREADS, TRTRI_SMEM);
   if (e != cudaSuccess) return e;
   for (int k0 = 0; k0 < count; k0 += TRTRI_MAXI) {
     TrtriBatch B;
     std::memset(&B, 0, sizeof(B));
-    long long total = 0, nflag = 0;
+    long long total = 0, nflag = 0, diag = 0;
+    double work = 0;  // tile products of the launch
+    int nqmax = 0;
     for (int k = k0; k < std::min(count, k0 + TRTRI_MAXI); ++k) {
       TrtriDev& I = B.inst[B.count];
       I.D = inst[k].D;
@@ -358,18 +388,40 @@ int block_trtri(const TrtriInst* inst, int count, int* flags, int* abort_flag, c
       if (I.n <= 0 || I.b <= 0) continue;
       nflag += (long long)I.n * I.nq * I.nq;
       total += (long long)I.n * I.nq * (I.nq + 1) / 2;
+      diag += (long long)I.n * I.nq;
+      work += (double)I.n * I.nq * I.nq * I.nq / 6;
+      nqmax = std::max(nqmax, I.nq);
       B.count++;
     }
+    // Columns when every CTA slot has at least COLUMN_WORK times the tile
+    // products of the longest column to do: tile by tile against column by
+    // column, 12 x 20 blocks of 1500 (4.3 times) 10.78 and 10.05 ms, 100 of
+    // 1500 (1.8) 4.55 and 4.18, 30 of 2500 (0.90) 5.95 and 5.62, 20 of 4000
+    // (0.95) 14.6 and 14.0, 40 of 1500 (0.72) 1.88 and 1.85; 10 of 6000 (0.71)
+    // 24.3 and 25.8, 14 of 4000 (0.66) 10.3 and 11.2, 20 of 1500 (0.36) 0.99 and
+    // 1.52.  Blocks of one or two tiles gain nothing (1200 of 128: 0.124, 0.130).
+    const int slots = std::max(1, occ) * device_sm_count();
+    const bool columns = nqmax > 2 && work >= COLUMN_WORK * (0.5 * nqmax * nqmax) * slots;
     if (total == 0) continue;
     if (total > INT32_MAX / 2) return cudaErrorInvalidValue;
-    B.total = (int)total;
+    B.total = (int)(columns ? diag : total);
+    B.zeros = columns ? 0 : 1;
+    B.nqmax = nqmax;
     B.flags = flags;
     B.counter = flags + nflag;
     B.abort_flag = abort_flag;
     if ((e = cudaMemsetAsync(flags, 0, (nflag + 1) * sizeof(int), s)) != cudaSuccess) return e;
-    bta::ProfScope _ps(bta::PROF_TRTRI, s);
-    const int grid = (int)std::min<long long>(total, (long long)std::max(1, occ) * device_sm_count());
-    block_trtri_kernel<<<grid, THREADS, TRTRI_SMEM, s>>>(B);
+    {
+      bta::ProfScope _ps(bta::PROF_TRTRI, s);
+      block_trtri_kernel<false><<<std::min(B.total, slots), THREADS, TRTRI_SMEM, s>>>(B);
+    }
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (!columns) continue;
+    B.total = (int)diag;  // as many columns
+    {
+      bta::ProfScope _ps(bta::PROF_TRTRI, s);
+      block_trtri_kernel<true><<<B.total, THREADS, TRTRI_SMEM, s>>>(B);
+    }
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   return cudaSuccess;
