@@ -904,6 +904,11 @@ int gemm_launch_i8(const std::vector<GemmProb>& probs, cudaStream_t stream, int*
   }
   uint8_t* w = static_cast<uint8_t*>(ws);
   std::vector<SliceGroup> groups;
+  // groups by their first operand: open addressing, at most half full (a group
+  // of block columns of small blocks has thousands of sides)
+  size_t slots = 4;
+  while (slots < 4 * probs.size()) slots *= 2;
+  std::vector<int> by_operand(slots, -1);
   std::vector<QProb> qp;
   for (const GemmProb& p : probs) {
     if (p.M <= 0 || p.N <= 0) continue;
@@ -950,9 +955,10 @@ int gemm_launch_i8(const std::vector<GemmProb>& probs, cudaStream_t stream, int*
       return eq;
     };
     auto plan = [&](SliceGroup& gr) {
-      for (const SliceGroup& o : groups)
-        if (same(o, gr)) {
-          gr = o;
+      size_t at = ((reinterpret_cast<uintptr_t>(gr.s[0].P) >> 3) * 0x9E3779B97F4A7C15ull >> 32) & (slots - 1);
+      for (; by_operand[at] >= 0; at = (at + 1) & (slots - 1))
+        if (same(groups[by_operand[at]], gr)) {
+          gr = groups[by_operand[at]];
           return;
         }
       if (reuse)
@@ -968,6 +974,7 @@ int gemm_launch_i8(const std::vector<GemmProb>& probs, cudaStream_t stream, int*
         gr.s[s].out = reinterpret_cast<int8_t*>(w);
         w += (size_t)gr.s[s].KT * gr.RB * A_BLOCK;
       }
+      by_operand[at] = (int)groups.size();
       groups.push_back(gr);
     };
     plan(ga);
