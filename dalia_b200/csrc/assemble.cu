@@ -123,14 +123,12 @@ __global__ void tip_final_kernel(int nparts, int a, const double* part, double p
 }
 
 // The four sums out[0 .. 3] = sum_row sum_e f(row, e) vals4[e][0 .. 3] over a
-// union pattern of ns rows, by a cluster of BI_CTAS CTAs: each takes a range of
+// union pattern of ns rows, by a cluster of CTAS CTAs: each takes a range of
 // rows, eight lanes per row (neighbouring entries, whose values are
 // contiguous), and CTA 0 adds the CTAs' sums in order.  The entries are
 // gathered, so latency bounds these kernels: one CTA per block with a thread
 // per row left most SMs idle (19 blocks of 289: 52 us, now 9 us).
-constexpr int BI_CTAS = 8;
-
-template <class F>
+template <int CTAS, class F>
 __device__ __forceinline__ void pattern_sums(int ns, const int* rowptr, const int* colidx, const double* vals4,
                                              double* out, F f) {
   __shared__ double red[8][4];
@@ -138,7 +136,7 @@ __device__ __forceinline__ void pattern_sums(int ns, const int* rowptr, const in
   namespace cg = cooperative_groups;
   const cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank(), tid = threadIdx.x, sub = tid & 7;
-  const int lo = (int)((long long)ns * rank / BI_CTAS), hi = (int)((long long)ns * (rank + 1) / BI_CTAS);
+  const int lo = (int)((long long)ns * rank / CTAS), hi = (int)((long long)ns * (rank + 1) / CTAS);
   const bool vec = (reinterpret_cast<uintptr_t>(vals4) & 15) == 0;
   double s[4] = {0.0, 0.0, 0.0, 0.0};
   for (int row = lo + (tid >> 3); row < hi; row += 32) {
@@ -176,42 +174,69 @@ __device__ __forceinline__ void pattern_sums(int ns, const int* rowptr, const in
   cl.sync();
   if (rank == 0 && tid < 4) {
     double t = 0.0;
-    for (int r = 0; r < BI_CTAS; ++r) t += cl.map_shared_rank(mine, r)[tid];
+    for (int r = 0; r < CTAS; ++r) t += cl.map_shared_rank(mine, r)[tid];
     out[tid] = t;
   }
   cl.sync();  // the CTAs' sums stay until they are read
 }
 
+// CTAs per cluster for that many units: as many as keep the launch within
+// per_sm CTAs per SM.  37 entries per row, us with 1, 2, 4 and 8 CTAs per unit,
+//               inner (11 per SM)      quad (5)          bilinear (4)
+//   19 x  289    26  20  16  16     24  19  16  16     27  20  17  16
+//   79 x  600    39  21  15  19     39  19  14  12     44  21  14  18
+//  199 x 1500   149  90  99  82     80  47  59  57     93  51  67  55
+//  499 x  600    78  83  87 108     48  60  55  67     54  59  66  81
+// 1999 x  100    57  70  97 184     42  53  70 114     50  58  80 135
+int cluster_ctas(long long units, int per_sm) {
+  int c = 1;
+  while (c < 8 && units * 2 * c <= (long long)per_sm * bta::device_sm_count()) c *= 2;
+  return c;
+}
+
+// One cluster per unit; k: the kernel with clusters of 1, 2, 4 and 8.
+template <class... P>
+struct UnitKernels {
+  void (*k[4])(P...);
+};
+template <class... P>
+void launch_units(long long units, int per_sm, cudaStream_t s, const UnitKernels<P...>& kernels, P... args) {
+  const int c = cluster_ctas(units, per_sm);
+  kernels.k[c == 8 ? 3 : c / 2]<<<(unsigned)(units * c), 256, 0, s>>>(args...);
+}
+
 // out[blk][v][w][K] = sum over the union pattern of sub-block (v, w) of block
 // blk of S[v ns + s][w ns + c] * K[s][c] (blk < n: diagonal block D_t; else
 // sub-diagonal block L_{blk-n}).  One cluster per (blk, v, w).
-__global__ void __cluster_dims__(BI_CTAS, 1, 1) __launch_bounds__(256)
+template <int CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(256)
     block_inner_kernel(int n, int ns, int nv, const int* rowptr, const int* colidx, const double* vals4,
                        const double* D, const double* L, double* out) {
-  const int unit = blockIdx.x / BI_CTAS;
+  const int unit = blockIdx.x / CTAS;
   const int blk = unit / (nv * nv), vw = unit % (nv * nv), v = vw / nv, w = vw % nv;
   const int b = nv * ns;
   const bool lower = blk >= n;
   const int t = lower ? blk - n : blk;
   const double* M = (lower ? L + (size_t)t * b * b : D + (size_t)t * b * b) + (size_t)v * ns * b + w * ns;
-  pattern_sums(ns, rowptr, colidx, vals4, out + (size_t)unit * 4,
+  pattern_sums<CTAS>(ns, rowptr, colidx, vals4, out + (size_t)unit * 4,
                [&](int row, int c) { return M[(size_t)row * b + c]; });
 }
 
 // out[blk][v][w][K] = x_{r,v}^T K x_{c,w} over the union pattern, where x_{t,v}
 // is variate v's segment of time step t, (r, c) = (t, t) for the diagonal
 // block t = blk < n and (t+1, t) for the sub-diagonal block t = blk - n.
-__global__ void __cluster_dims__(BI_CTAS, 1, 1) __launch_bounds__(256)
+template <int CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(256)
     block_quad_kernel(int n, int ns, int nv, const int* rowptr, const int* colidx, const double* vals4,
                       const double* x, double* out) {
-  const int unit = blockIdx.x / BI_CTAS;
+  const int unit = blockIdx.x / CTAS;
   const int blk = unit / (nv * nv), vw = unit % (nv * nv), v = vw / nv, w = vw % nv;
   const int b = nv * ns;
   const bool lower = blk >= n;
   const int t = lower ? blk - n : blk;
   const double* xr = x + (size_t)(lower ? t + 1 : t) * b + v * ns;
   const double* xc = x + (size_t)t * b + w * ns;
-  pattern_sums(ns, rowptr, colidx, vals4, out + (size_t)unit * 4, [&](int row, int c) { return xr[row] * xc[c]; });
+  pattern_sums<CTAS>(ns, rowptr, colidx, vals4, out + (size_t)unit * 4, [&](int row, int c) { return xr[row] * xc[c]; });
 }
 
 // out[blockIdx] partial of sum_e w[e] * base[idx[e]]
@@ -365,17 +390,18 @@ __global__ void __launch_bounds__(256) poisson_terms_kernel(int64_t m, const dou
 // out[blk][K] = u_t^T K x_t (diagonal block t = blk < n) or
 // u_{t+1}^T K x_t + u_t^T K x_{t+1} (sub-diagonal block t = blk - n): the
 // bilinear form u^T (E (x) K) x of the symmetric Kronecker block pair.
-__global__ void __cluster_dims__(BI_CTAS, 1, 1) __launch_bounds__(256)
+template <int CTAS>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(256)
     block_bilinear_kernel(int n, int b, const int* rowptr, const int* colidx, const double* vals4, const double* u,
                           const double* x, double* out) {
-  const int blk = blockIdx.x / BI_CTAS;
+  const int blk = blockIdx.x / CTAS;
   const bool lower = blk >= n;
   const int t = lower ? blk - n : blk;
   const double* ur = u + (size_t)(lower ? t + 1 : t) * b;
   const double* xc = x + (size_t)t * b;
   const double* ur2 = u + (size_t)t * b;
   const double* xc2 = x + (size_t)(t + 1) * b;
-  pattern_sums(b, rowptr, colidx, vals4, out + (size_t)blk * 4, [&](int row, int c) {
+  pattern_sums<CTAS>(b, rowptr, colidx, vals4, out + (size_t)blk * 4, [&](int row, int c) {
     return ur[row] * xc[c] + (lower ? ur2[row] * xc2[c] : 0.0);
   });
 }
@@ -485,8 +511,9 @@ int bta_block_inner_mv(void* stream, int64_t n, int64_t ns, int64_t nv, const in
   if (n < 1 || ns < 1 || nv < 1 || !out || !D || (n > 1 && !L)) return BTA_ERR_INVALID;
   {
     bta::ProfScope _ps(bta::PROF_OTHER, (cudaStream_t)stream);
-    block_inner_kernel<<<(int)((2 * n - 1) * nv * nv * BI_CTAS), 256, 0, (cudaStream_t)stream>>>(
-        (int)n, (int)ns, (int)nv, rowptr, colidx, vals4, D, L, out);
+    launch_units((2 * n - 1) * nv * nv, 11, (cudaStream_t)stream,
+                 {block_inner_kernel<1>, block_inner_kernel<2>, block_inner_kernel<4>, block_inner_kernel<8>}, (int)n,
+                 (int)ns, (int)nv, rowptr, colidx, vals4, D, L, out);
   }
   return cudaGetLastError() == cudaSuccess ? BTA_OK : BTA_ERR_CUDA;
 }
@@ -501,8 +528,9 @@ int bta_block_quad_mv(void* stream, int64_t n, int64_t ns, int64_t nv, const int
   if (n < 1 || ns < 1 || nv < 1 || !out || !x) return BTA_ERR_INVALID;
   {
     bta::ProfScope _ps(bta::PROF_OTHER, (cudaStream_t)stream);
-    block_quad_kernel<<<(int)((2 * n - 1) * nv * nv * BI_CTAS), 256, 0, (cudaStream_t)stream>>>(
-        (int)n, (int)ns, (int)nv, rowptr, colidx, vals4, x, out);
+    launch_units((2 * n - 1) * nv * nv, 5, (cudaStream_t)stream,
+                 {block_quad_kernel<1>, block_quad_kernel<2>, block_quad_kernel<4>, block_quad_kernel<8>}, (int)n,
+                 (int)ns, (int)nv, rowptr, colidx, vals4, x, out);
   }
   return cudaGetLastError() == cudaSuccess ? BTA_OK : BTA_ERR_CUDA;
 }
@@ -583,8 +611,9 @@ int bta_block_bilinear(void* stream, int64_t n, int64_t b, const int* rowptr, co
   if (n < 1 || b < 1 || !rowptr || !colidx || !vals4 || !u || !x || !out) return BTA_ERR_INVALID;
   {
     bta::ProfScope _ps(bta::PROF_OTHER, (cudaStream_t)stream);
-    block_bilinear_kernel<<<(int)(2 * n - 1) * BI_CTAS, 256, 0, (cudaStream_t)stream>>>((int)n, (int)b, rowptr, colidx, vals4,
-                                                                            u, x, out);
+    launch_units(2 * n - 1, 4, (cudaStream_t)stream,
+                 {block_bilinear_kernel<1>, block_bilinear_kernel<2>, block_bilinear_kernel<4>, block_bilinear_kernel<8>},
+                 (int)n, (int)b, rowptr, colidx, vals4, u, x, out);
   }
   return cudaGetLastError() == cudaSuccess ? BTA_OK : BTA_ERR_CUDA;
 }
