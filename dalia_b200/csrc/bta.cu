@@ -12,6 +12,7 @@
 #include "../../include/dalia_bta.h"
 #include "bta_internal.cuh"
 #include "gemm.cuh"
+#include "lists.cuh"
 #include "panel.cuh"
 #include "prof.cuh"
 #include "tune.cuh"
@@ -151,6 +152,13 @@ struct PanelSpec {
   double* Ttip = nullptr;
 };
 
+int upload_tasks(const std::vector<int4>& t, int4** d) {
+  const cudaError_t e = upload_list(reinterpret_cast<void**>(d), t.data(), t.size() * sizeof(int4));
+  if (e == cudaSuccess) return BTA_OK;
+  cudaGetLastError();
+  return e == cudaErrorMemoryAllocation ? BTA_ERR_ALLOC : BTA_ERR_CUDA;
+}
+
 // Cached device task list of a panel batch with the given instance shapes
 // and queue lookahead.
 int get_tasks(bta_context* h, const std::vector<PanelInst>& insts, int lookahead, int order, const int4** out,
@@ -168,9 +176,8 @@ int get_tasks(bta_context* h, const std::vector<PanelInst>& insts, int lookahead
     panel_tasks(insts, t, lookahead, order);
     int4* d = nullptr;
     if (!t.empty()) {
-      if (cudaMalloc(&d, t.size() * sizeof(int4)) != cudaSuccess) return BTA_ERR_ALLOC;
-      if (cudaMemcpy(d, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess)
-        return BTA_ERR_CUDA;
+      const int rc = upload_tasks(t, &d);
+      if (rc) return rc;
     }
     it = h->tasks.emplace(key, std::make_pair(d, (int)t.size())).first;
   }
@@ -424,8 +431,7 @@ int run_factor_persist(bta_context* h, int count, const int64_t* n, const int64_
     std::vector<int4> t;
     panel_tasks_persist(shapes, nn, col_start, t, lookahead, order);
     int4* d = nullptr;
-    if (cudaMalloc(&d, t.size() * sizeof(int4)) != cudaSuccess) return BTA_ERR_ALLOC;
-    if (cudaMemcpy(d, t.data(), t.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess) return BTA_ERR_CUDA;
+    if ((rc = upload_tasks(t, &d))) return rc;
     it = h->tasks.emplace(key, std::make_pair(d, (int)t.size())).first;
   }
   PanelBatch B;

@@ -38,6 +38,7 @@
 #include <vector>
 
 #include "gemm.cuh"
+#include "lists.cuh"
 #include "prof.cuh"
 #include "tune.cuh"
 
@@ -846,13 +847,8 @@ const int* tile_list(I8Plans* plans, const QBatch& b, int total, int grid, cudaS
   }
   const std::vector<int> list = deal_tiles<BN>(b, total, grid);
   int* d = nullptr;
-  if (cudaMalloc(&d, list.size() * sizeof(int)) != cudaSuccess) {
+  if (upload_list(reinterpret_cast<void**>(&d), list.data(), list.size() * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
-    return nullptr;
-  }
-  if (cudaMemcpy(d, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(d);
     return nullptr;
   }
   plans->by_shape.emplace(std::move(key), d);
