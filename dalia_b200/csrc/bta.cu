@@ -270,8 +270,10 @@ int run_panels(bta_context* h, const std::vector<PanelSpec>& specs, Carve& cv) {
 }
 
 // Whether an FP64 factorisation runs as one launch: by default when its
-// workspace (the tile inverses and flags of every block column) is at most
-// PERSIST_WS; DALIA_B200_PANEL_PERSIST=1 / 0 forces it on / off.  Measured on
+// workspace (the tile inverses and flags of every block column, 64/b of the
+// diagonal blocks' size) is at most PERSIST_WS and, where the handle's has to
+// grow for it, at most a quarter of the free memory: a column launch does with
+// one column's, and the caller may need the rest.  DALIA_B200_PANEL_PERSIST=1 / 0 forces it on / off.  Measured on
 // B200 against one launch per block column, best candidates of each: 10
 // blocks of 300, one matrix 1.32 -> 1.05 ms, 12 matrices 1.99 -> 1.57; 24 of
 // 617 6.5 -> 5.5; 20 of 1500 13.5 -> 10.3; 10 of 1500, 12 matrices 33.7 ->
@@ -279,11 +281,18 @@ int run_panels(bta_context* h, const std::vector<PanelSpec>& specs, Carve& cv) {
 // column ends; a column launch starts with them, each a whole block's sum,
 // before its chain can begin.)
 constexpr size_t PERSIST_WS = size_t(2) << 30;
-bool persist_enabled(size_t bytes) {
+bool persist_enabled(const bta_context* h, size_t bytes) {
   const char* e = std::getenv("DALIA_B200_PANEL_PERSIST");
   if (e && std::strcmp(e, "1") == 0) return true;
   if (e && std::strcmp(e, "0") == 0) return false;
-  return bytes <= PERSIST_WS;
+  if (bytes > PERSIST_WS) return false;
+  if (bytes <= h->ws_bytes) return true;
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return bytes <= (free + h->ws_bytes) / 4;
 }
 
 // Per-instance part of the column descriptors of a whole factorisation, and
@@ -595,8 +604,8 @@ int bta_pobtaf_batched_ex(bta_handle_t h, int count, const int64_t* n, const int
     if (rc) return rc;
   }
   // FP64 with every arrow tip inside the panel: the whole factorisation in one
-  // launch, unless its workspace is too large or cannot be had
-  bool persist = !split && count <= PANEL_MAXI && persist_enabled(persist_ws_bytes(count, n, b, a));
+  // launch, unless its workspace is too large
+  bool persist = !split && count <= PANEL_MAXI && persist_enabled(h, persist_ws_bytes(count, n, b, a));
   for (int k = 0; k < count; ++k) persist = persist && a[k] <= 64;
   if (persist) {
     rc = run_factor_persist(h, count, n, b, a, D, L, Ab, T);

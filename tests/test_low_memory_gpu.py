@@ -1,0 +1,66 @@
+"""Calls on a GPU that is nearly full do with the workspace that one block
+column needs."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+MB = 1 << 20
+
+
+def _bta(n, b, a, seed):
+    import torch
+
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, dtype=torch.float64, device="cuda", generator=g)  # noqa: E731
+    D = rnd(n, b, b) / (4 * b)
+    D = D + D.transpose(1, 2) + 4 * torch.eye(b, dtype=torch.float64, device="cuda")
+    return [D.contiguous(), rnd(max(n - 1, 0), b, b) / (2 * b), rnd(n, a, b) / (4 * b),
+            n * torch.eye(a, dtype=torch.float64, device="cuda")]
+
+
+def _args(n, b, a, m):
+    one, ptr = ctypes.c_int64 * 1, ctypes.c_void_p * 1
+    return [1, one(n), one(b), one(a)] + [ptr(x.data_ptr() if x.numel() else None) for x in m]
+
+
+def _fill(leave):
+    """Takes the GPU's memory but for `leave` bytes."""
+    import torch
+
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free, _ = torch.cuda.mem_get_info()
+    return torch.empty(max(0, free - leave), dtype=torch.uint8, device="cuda")
+
+
+def _err(got, ref):
+    return max(float((x - y).norm() / y.norm()) for x, y in zip(got, ref) if y.numel())
+
+
+def test_factorisation_takes_at_most_a_quarter_of_what_is_free(monkeypatch):
+    import torch
+
+    from dalia_b200 import _lib
+
+    monkeypatch.delenv("DALIA_B200_PANEL_PERSIST", raising=False)
+    lib = _lib.load()
+    n, b, a = 8000, 64, 2  # tile inverses of all block columns: 250 MB
+    m = _bta(n, b, a, 1)
+    got, ref = [x.clone() for x in m], [x.clone() for x in m]
+    info = ctypes.c_int64(-1)
+    wide = _lib.Handle()
+    _lib.check(lib.bta_pobtaf_batched(wide.bind_stream(), *_args(n, b, a, ref), ctypes.byref(info)), "pobtaf")
+    assert wide.workspace_bytes() > 200 * MB
+    del wide
+    h = _lib.Handle()
+    filler = _fill(600 * MB)
+    _lib.check(lib.bta_pobtaf_batched(h.bind_stream(), *_args(n, b, a, got), ctypes.byref(info)), "pobtaf")
+    held = h.workspace_bytes()
+    del filler
+    torch.cuda.empty_cache()
+    assert held < 150 * MB
+    # one factorisation in two launch orders: the same sums
+    assert _err(got, ref) <= 1e-12
