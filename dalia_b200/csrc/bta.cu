@@ -65,13 +65,20 @@ int ensure_ws2(bta_context* h, size_t bytes) {
   return BTA_OK;
 }
 
-// Grouped GEMM in the requested arithmetic on the handle's stream.
+// Grouped GEMM in the requested arithmetic on the handle's stream.  The
+// problems of a group are independent: where memory for the digit images of
+// all of them cannot be had, the group is launched in halves.
 int run_gemm(bta_context* h, const std::vector<GemmProb>& pr, int precision) {
   if (precision == BTA_PREC_TF32X3) return gemm_launch_tc(pr, h->stream, h->ctl) ? BTA_ERR_CUDA : BTA_OK;
   if (precision == BTA_PREC_I8SLICE) {
     size_t need = 0;
     if (gemm_launch_i8(pr, h->stream, h->ctl, nullptr, 0, &need)) return BTA_ERR_INVALID;
     int rc = ensure_ws2(h, need);
+    if (rc == BTA_ERR_ALLOC && pr.size() > 1) {
+      const auto mid = pr.begin() + pr.size() / 2;
+      rc = run_gemm(h, std::vector<GemmProb>(pr.begin(), mid), precision);
+      return rc ? rc : run_gemm(h, std::vector<GemmProb>(mid, pr.end()), precision);
+    }
     if (rc) return rc;
     return gemm_launch_i8(pr, h->stream, h->ctl, h->ws2, h->ws2_bytes, nullptr, &h->i8plans) ? BTA_ERR_CUDA : BTA_OK;
   }
@@ -80,19 +87,21 @@ int run_gemm(bta_context* h, const std::vector<GemmProb>& pr, int precision) {
 
 // Two grouped GEMMs, one after the other, the A sides of the second partly
 // equal to B sides of the first (operands that the first does not write): the
-// 8-bit-slice arithmetic cuts those once.
+// 8-bit-slice arithmetic cuts those once, where the images of both fit.
 int run_gemm_pair(bta_context* h, const std::vector<GemmProb>& p1, const std::vector<GemmProb>& p2, int precision) {
-  if (precision != BTA_PREC_I8SLICE || p1.empty() || p2.empty()) {
+  auto apart = [&]() {
     int rc = BTA_OK;
     if (!p1.empty()) rc = run_gemm(h, p1, precision);
     if (!rc && !p2.empty()) rc = run_gemm(h, p2, precision);
     return rc;
-  }
+  };
+  if (precision != BTA_PREC_I8SLICE || p1.empty() || p2.empty()) return apart();
   size_t need1 = 0, need2 = 0;
   if (gemm_launch_i8(p1, h->stream, h->ctl, nullptr, 0, &need1) ||
       gemm_launch_i8(p2, h->stream, h->ctl, nullptr, 0, &need2))
     return BTA_ERR_INVALID;
-  int rc = ensure_ws2(h, need1 + need2);
+  const int rc = ensure_ws2(h, need1 + need2);
+  if (rc == BTA_ERR_ALLOC) return apart();
   if (rc) return rc;
   std::vector<I8Side> sides;
   if (gemm_launch_i8(p1, h->stream, h->ctl, h->ws2, need1, nullptr, &h->i8plans, &sides)) return BTA_ERR_CUDA;
@@ -885,19 +894,28 @@ int bta_pobtasi_batched_v(bta_handle_t h, int count, const int64_t* n, const int
   // workspace for large blocks and puts a whole inversion of small blocks
   // into one launch.  The recurrence itself is then two dependent launches
   // per block column instead of three.
-  const int64_t want = std::max<int64_t>(1, (int64_t)std::ceil(12.0 * device_sm_count() / step_tiles));
+  // Where that much workspace cannot be had, one block column at a time.
+  int64_t want = std::max<int64_t>(1, (int64_t)std::ceil(12.0 * device_sm_count() / step_tiles));
   std::vector<int64_t> group(count, 1);
   for (int k = 0; k < count; ++k) {
-    const size_t bb = (size_t)b[k] * b[k], ab = (size_t)a[k] * b[k];
-    group[k] = std::min(want, chunk[k] ? chunk[k] : n[k]);
+    const size_t bb = (size_t)b[k] * b[k];
     // block inverses of a chunk only when not supplied
     nflags += chunk[k] ? block_trtri_flags((int)chunk[k], (int)b[k]) : 0;
     ntipflags += a[k] > 0 ? block_trtri_flags(1, (int)a[k]) : 0;
-    need += (chunk[k] ? align_up(chunk[k] * bb * 8) : 0) + align_up(group[k] * bb * 8) +
-            align_up(group[k] * ab * 8 + 8) + align_up((size_t)a[k] * a[k] * 8 + 8) + 4 * kAlign;
+    need += (chunk[k] ? align_up(chunk[k] * bb * 8) : 0) + align_up((size_t)a[k] * a[k] * 8 + 8) + 4 * kAlign;
   }
   need += align_up(std::max(nflags, ntipflags) * sizeof(int));
-  int rc = ensure_ws(h, need);
+  int rc = BTA_ERR_ALLOC;
+  for (;; want = 1) {
+    size_t all = need;
+    for (int k = 0; k < count; ++k) {
+      const size_t bb = (size_t)b[k] * b[k], ab = (size_t)a[k] * b[k];
+      group[k] = std::min(want, chunk[k] ? chunk[k] : n[k]);
+      all += align_up(group[k] * bb * 8) + align_up(group[k] * ab * 8 + 8);
+    }
+    rc = ensure_ws(h, all);
+    if (rc != BTA_ERR_ALLOC || want == 1) break;
+  }
   if (rc) return rc;
   cudaStream_t s = h->stream;
   Carve cv{h->ws};

@@ -64,3 +64,40 @@ def test_factorisation_takes_at_most_a_quarter_of_what_is_free(monkeypatch):
     assert held < 150 * MB
     # one factorisation in two launch orders: the same sums
     assert _err(got, ref) <= 1e-12
+
+
+@pytest.mark.parametrize("leave", [110, 34])
+def test_selected_inversion_in_parts(leave):
+    """8-bit slices of blocks of 1000 with supplied inverses: the digit images of
+    a group of five block columns take 160 MB, those of a step's two launches
+    32, those of one product 16."""
+    import torch
+
+    from dalia_b200 import _lib
+
+    lib = _lib.load()
+    n, b, a = 6, 1000, 0
+    m = _bta(n, b, a, 2)
+    info = ctypes.c_int64(-1)
+    h = _lib.handle()
+    _lib.check(lib.bta_pobtaf_batched(h.bind_stream(), *_args(n, b, a, m), ctypes.byref(info)), "pobtaf")
+    V = torch.empty_like(m[0])
+    one, ptr = ctypes.c_int64 * 1, ctypes.c_void_p * 1
+    _lib.check(lib.bta_block_inverses(h.bind_stream(), 1, one(n), one(b), ptr(m[0].data_ptr()), ptr(V.data_ptr())),
+               "inverses")
+    got, ref = [x.clone() for x in m], [x.clone() for x in m]
+
+    def run(h, w):
+        rc = lib.bta_pobtasi_batched_v(h.bind_stream(), *_args(n, b, a, w), ptr(V.data_ptr()), _lib.BTA_PREC_I8SLICE)
+        return rc or lib.bta_get_status(h.bind_stream(), ctypes.byref(info))
+
+    wide, h = _lib.Handle(), _lib.Handle()
+    assert run(wide, ref) == 0
+    del wide
+    filler = _fill(leave * MB)
+    rc = run(h, got)
+    del filler, h
+    torch.cuda.empty_cache()
+    assert rc == 0
+    # the same digits and the same integer sums, launched in other groups
+    assert _err(got, ref) <= 1e-12
