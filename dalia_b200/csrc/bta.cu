@@ -28,8 +28,8 @@ struct bta_context {
   size_t ws2_bytes = 0;
   int* ctl = nullptr;  // [0] abort flag, [1] scratch; ctl+2 (8-aligned): info (u64)
   double* scal = nullptr;
-  std::map<std::vector<int>, std::pair<int4*, int>> tasks;
-  I8Plans i8plans;  // tile lists of the 8-bit-slice GEMM's launch shapes
+  ShapeLists tasks;    // task queues of the factorisation's launch shapes
+  ShapeLists i8lists;  // tile lists of the 8-bit-slice GEMM's
 };
 
 namespace {
@@ -80,7 +80,7 @@ int run_gemm(bta_context* h, const std::vector<GemmProb>& pr, int precision) {
       return rc ? rc : run_gemm(h, std::vector<GemmProb>(mid, pr.end()), precision);
     }
     if (rc) return rc;
-    return gemm_launch_i8(pr, h->stream, h->ctl, h->ws2, h->ws2_bytes, nullptr, &h->i8plans) ? BTA_ERR_CUDA : BTA_OK;
+    return gemm_launch_i8(pr, h->stream, h->ctl, h->ws2, h->ws2_bytes, nullptr, &h->i8lists) ? BTA_ERR_CUDA : BTA_OK;
   }
   return gemm_launch(pr, h->stream) ? BTA_ERR_CUDA : BTA_OK;
 }
@@ -104,8 +104,8 @@ int run_gemm_pair(bta_context* h, const std::vector<GemmProb>& p1, const std::ve
   if (rc == BTA_ERR_ALLOC) return apart();
   if (rc) return rc;
   std::vector<I8Side> sides;
-  if (gemm_launch_i8(p1, h->stream, h->ctl, h->ws2, need1, nullptr, &h->i8plans, &sides)) return BTA_ERR_CUDA;
-  return gemm_launch_i8(p2, h->stream, h->ctl, h->ws2 + need1, need2, nullptr, &h->i8plans, nullptr, &sides)
+  if (gemm_launch_i8(p1, h->stream, h->ctl, h->ws2, need1, nullptr, &h->i8lists, &sides)) return BTA_ERR_CUDA;
+  return gemm_launch_i8(p2, h->stream, h->ctl, h->ws2 + need1, need2, nullptr, &h->i8lists, nullptr, &sides)
              ? BTA_ERR_CUDA
              : BTA_OK;
 }
@@ -161,8 +161,8 @@ struct PanelSpec {
   double* Ttip = nullptr;
 };
 
-int upload_tasks(const std::vector<int4>& t, int4** d) {
-  const cudaError_t e = upload_list(reinterpret_cast<void**>(d), t.data(), t.size() * sizeof(int4));
+int add_tasks(bta_context* h, std::vector<int>&& key, const std::vector<int4>& t, const ShapeLists::List** out) {
+  const cudaError_t e = h->tasks.add(std::move(key), t.data(), (int)t.size(), t.size() * sizeof(int4), h->stream, out);
   if (e == cudaSuccess) return BTA_OK;
   cudaGetLastError();
   return e == cudaErrorMemoryAllocation ? BTA_ERR_ALLOC : BTA_ERR_CUDA;
@@ -179,19 +179,15 @@ int get_tasks(bta_context* h, const std::vector<PanelInst>& insts, int lookahead
     key.push_back((I.L != nullptr ? 1 : 0) | (I.Ttip != nullptr ? 2 : 0) | (I.Lprev != nullptr ? 4 : 0) |
                   (I.Abprev != nullptr ? 8 : 0));
   }
-  auto it = h->tasks.find(key);
-  if (it == h->tasks.end()) {
+  const ShapeLists::List* l = h->tasks.find(key, h->stream);
+  if (!l) {
     std::vector<int4> t;
     panel_tasks(insts, t, lookahead, order);
-    int4* d = nullptr;
-    if (!t.empty()) {
-      const int rc = upload_tasks(t, &d);
-      if (rc) return rc;
-    }
-    it = h->tasks.emplace(key, std::make_pair(d, (int)t.size())).first;
+    const int rc = add_tasks(h, std::move(key), t, &l);
+    if (rc) return rc;
   }
-  *out = it->second.first;
-  *count = it->second.second;
+  *out = static_cast<const int4*>(l->d);
+  *count = l->n;
   return BTA_OK;
 }
 
@@ -444,19 +440,17 @@ int run_factor_persist(bta_context* h, int count, const int64_t* n, const int64_
     key.push_back((int)a[k]);
     key.push_back(nn[k]);
   }
-  auto it = h->tasks.find(key);
-  if (it == h->tasks.end()) {
+  const ShapeLists::List* l = h->tasks.find(key, s);
+  if (!l) {
     std::vector<int4> t;
     panel_tasks_persist(shapes, nn, col_start, t, lookahead, order);
-    int4* d = nullptr;
-    if ((rc = upload_tasks(t, &d))) return rc;
-    it = h->tasks.emplace(key, std::make_pair(d, (int)t.size())).first;
+    if ((rc = add_tasks(h, std::move(key), t, &l))) return rc;
   }
   PanelBatch B;
   std::memset(&B, 0, sizeof(B));
   B.ninst = count;
-  B.ntasks = it->second.second;
-  B.tasks = it->second.first;
+  B.ntasks = l->n;
+  B.tasks = static_cast<const int4*>(l->d);
   B.counter = batch_counter;
   B.sm_words = alone ? batch_counter + 4 : nullptr;
   B.abort_flag = h->ctl;
@@ -560,8 +554,6 @@ int bta_destroy(bta_handle_t h) {
   DeviceGuard dg_(h);
   if (!h) return BTA_ERR_INVALID;
   cudaStreamSynchronize(h->stream);
-  for (auto& kv : h->tasks) cudaFree(kv.second.first);
-  for (auto& kv : h->i8plans.by_shape) cudaFree(kv.second);
   if (h->ws) cudaFree(h->ws);
   if (h->ws2) cudaFree(h->ws2);
   cudaFree(h->ctl);

@@ -12,7 +12,6 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
-#include <map>
 #include <vector>
 
 namespace bta {
@@ -77,12 +76,7 @@ struct I8Side {
   } s[3];
 };
 
-// Tile lists of the 8-bit-slice GEMM's launches by launch shape, in device
-// memory (gemm_i8.cu), owned by a handle; at most I8_PLANS_MAX of them.
-struct I8Plans {
-  std::map<std::vector<int>, int*> by_shape;
-};
-constexpr size_t I8_PLANS_MAX = 256;
+class ShapeLists;  // lists.cuh
 
 // The same problems with 8-bit digit products accumulated exactly in INT32
 // (gemm_i8.cu).  With ws == nullptr only *ws_needed (bytes of workspace for
@@ -90,9 +84,9 @@ constexpr size_t I8_PLANS_MAX = 256;
 // record: receives the B sides of this launch (their images stay where they
 // are in ws).  reuse: sides recorded by an earlier launch whose operands and
 // images have not been written since; a side equal to one of them is not cut
-// again.  plans: the caller's cache of tile lists.
+// again.  lists: the caller's tile lists by launch shape.
 int gemm_launch_i8(const std::vector<GemmProb>& probs, cudaStream_t stream, int* abort_flag, void* ws,
-                   size_t ws_bytes, size_t* ws_needed, I8Plans* plans = nullptr,
+                   size_t ws_bytes, size_t* ws_needed, ShapeLists* lists = nullptr,
                    std::vector<I8Side>* record = nullptr, const std::vector<I8Side>* reuse = nullptr);
 
 inline GemmProb gemm_prob(double* C, int ldc, int M, int N, double beta, int cflags = 0) {

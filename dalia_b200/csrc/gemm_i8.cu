@@ -823,12 +823,12 @@ std::vector<int> deal_tiles(const QBatch& b, int total, int grid) {
   return list;
 }
 
-// The device list of a launch's tiles, from the cache or made now; nullptr
-// (tiles c, c + grid, ...) without a cache, when it cannot be had, or while
-// the stream is being captured and the shape is new.
+// The device list of a launch's tiles, kept or made now; nullptr (tiles c,
+// c + grid, ...) without a place to keep it, when it cannot be had, or while the
+// stream is being captured and the shape is new.
 template <int BN>
-const int* tile_list(I8Plans* plans, const QBatch& b, int total, int grid, cudaStream_t stream) {
-  if (!plans) return nullptr;
+const int* tile_list(ShapeLists* lists, const QBatch& b, int total, int grid, cudaStream_t stream) {
+  if (!lists) return nullptr;
   std::vector<int> key{BN, grid};
   for (int k = 0; k < b.count; ++k) {
     const QProb& p = b.p[k];
@@ -836,29 +836,22 @@ const int* tile_list(I8Plans* plans, const QBatch& b, int total, int grid, cudaS
     for (int s = 0; s < p.nseg; ++s) key.insert(key.end(), {p.seg[s].K, p.seg[s].kflags});
     if (p.tmn >= (1 << TILE_BITS) || p.tnn >= (1 << TILE_BITS)) return nullptr;
   }
-  auto it = plans->by_shape.find(key);
-  if (it != plans->by_shape.end()) return it->second;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return nullptr;
-  if (plans->by_shape.size() >= I8_PLANS_MAX) {
-    cudaStreamSynchronize(stream);  // launches that read a list end first
-    for (auto& e : plans->by_shape) cudaFree(e.second);
-    plans->by_shape.clear();
+  const ShapeLists::List* l = lists->find(key, stream);
+  if (!l) {
+    if (is_capturing(stream)) return nullptr;
+    const std::vector<int> list = deal_tiles<BN>(b, total, grid);
+    if (lists->add(std::move(key), list.data(), (int)list.size(), list.size() * sizeof(int), stream, &l) != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
   }
-  const std::vector<int> list = deal_tiles<BN>(b, total, grid);
-  int* d = nullptr;
-  if (upload_list(reinterpret_cast<void**>(&d), list.data(), list.size() * sizeof(int)) != cudaSuccess) {
-    cudaGetLastError();
-    return nullptr;
-  }
-  plans->by_shape.emplace(std::move(key), d);
-  return d;
+  return static_cast<const int*>(l->d);
 }
 
 template <int BN>
-void launch_tiles(I8Plans* plans, const QBatch& b, int total, int* abort_flag, cudaStream_t stream) {
+void launch_tiles(ShapeLists* lists, const QBatch& b, int total, int* abort_flag, cudaStream_t stream) {
   const int grid = std::min(total, device_sm_count());
-  const int* list = tile_list<BN>(plans, b, total, grid, stream);
+  const int* list = tile_list<BN>(lists, b, total, grid, stream);
   bta::ProfScope _ps(bta::PROF_GEMM, stream);
   gemm_i8_kernel<BN><<<grid, QTHREADS, QTile<BN>::SMEM_BYTES, stream>>>(b, total, list, abort_flag);
 }
@@ -866,7 +859,7 @@ void launch_tiles(I8Plans* plans, const QBatch& b, int total, int* abort_flag, c
 }  // namespace
 
 int gemm_launch_i8(const std::vector<GemmProb>& probs, cudaStream_t stream, int* abort_flag, void* ws,
-                   size_t ws_bytes, size_t* ws_needed, I8Plans* plans, std::vector<I8Side>* record,
+                   size_t ws_bytes, size_t* ws_needed, ShapeLists* lists, std::vector<I8Side>* record,
                    const std::vector<I8Side>* reuse) {
   // workspace: per problem the exponents of its rows and columns, per segment
   // the digit images of both operands
@@ -1026,8 +1019,8 @@ int gemm_launch_i8(const std::vector<GemmProb>& probs, cudaStream_t stream, int*
     }
     b.tile_start[b.count] = total;
     if (total > 0) {
-      if (BN == 64) launch_tiles<64>(plans, b, total, abort_flag, stream);
-      else launch_tiles<32>(plans, b, total, abort_flag, stream);
+      if (BN == 64) launch_tiles<64>(lists, b, total, abort_flag, stream);
+      else launch_tiles<32>(lists, b, total, abort_flag, stream);
     }
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
