@@ -479,9 +479,9 @@ int sweep_inv_steps(int count, const int* n, const int* b, const int* a, const d
     bsum += b[k];
     bmax = std::max(bmax, b[k]);
   }
-  // candidates: a CTA per SM, per two SMs (a quicker barrier, for small
-  // blocks), or two per SM (more loads in flight)
-  TuneLaunch tl("sweep", {count, trans, bsum, bmax, s1 - s0}, 3, s, 1);
+  // candidates: a CTA per SM, or per two SMs (a quicker barrier, for small
+  // blocks); two on an SM do not fit (512 threads of 124 registers)
+  TuneLaunch tl("sweep", {count, trans, bsum, bmax, s1 - s0}, 2, s, 1);
   const int cand = tl.choice();
   PSweep P;
   std::memset(&P, 0, sizeof(P));
@@ -515,14 +515,10 @@ int sweep_inv_steps(int count, const int* n, const int* b, const int* a, const d
   P.bar = reinterpret_cast<unsigned*>(work + off);
   if (cudaMemsetAsync(P.bar, 0, 2 * sizeof(unsigned), s) != cudaSuccess) return cudaErrorUnknown;
   auto kernel = bytes > PS_BIG_BYTES ? sweep_persist_kernel<true> : sweep_persist_kernel<false>;
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, PS_THREADS, 0) != cudaSuccess ||
-      occ <= 0)
-    return cudaErrorUnknown;
   const int sms = device_sm_count();
   // no more CTAs than there are groups of 8 rows, or strips
   const int most = std::max(1, trans == 0 ? (P.units + 7) / 8 : P.units);
-  const int grid = std::min(most, cand == 0 ? sms : cand == 1 ? std::max(1, sms / 2) : std::min(occ, 2) * sms);
+  const int grid = std::min(most, cand == 0 ? sms : std::max(1, sms / 2));
   void* args[] = {&P};
   bta::ProfScope _ps(bta::PROF_SWEEP, s);
   return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(kernel), dim3(grid),

@@ -24,7 +24,7 @@ namespace bta {
 constexpr int TUNE_REPS = 2;
 // Part of every key: decisions read from a file were made for these kernels
 // and these meanings of the candidates.  Raised when either changes.
-constexpr int TUNE_VERSION = 2;
+constexpr int TUNE_VERSION = 3;
 
 class TuneLaunch {
  public:
