@@ -690,24 +690,31 @@ int bta_pobtaf(bta_handle_t h, int64_t n, int64_t b, int64_t a, double* D, doubl
 }
 
 // Whether a sweep of these instances is faster through block inverses made
-// here chunk by chunk (b^3/3 flops per block on the tensor cores, then n
-// bandwidth-bound steps of the persistent sweep) than through the tile-task
-// sweep (n ceil(b/64) dependent 64-row links per instance, instances in
-// parallel).  Model: ~10 us per link, ~2 TB/s for the tile sweep's reads;
-// ~20 TF/s for the block inverses, ~15 us per persistent step.
-bool sweep_by_inverses(int count, const int64_t* n, const int64_t* b, const int64_t* a) {
-  double chain = 0, tile_bytes = 0, inv_flops = 0, inv_bytes = 0;
-  int64_t maxn = 0;
+// here chunk by chunk (b^3/3 flops per block on the tensor cores, then n steps
+// of the persistent sweep) than through the tile-task sweep (n ceil(b/64)
+// dependent 64-row links per instance, instances in parallel, each with launches
+// of its own).  Constants fitted to both sides of 358 sizes (n 3 to 100, b 20 to
+// 4000, 1 to 30 instances); the choice is within 5 % of the better side in all
+// but 11 of them.  Tile sweep and inverses, ms a sweep: 10 blocks of 192 0.134
+// and 0.113, of 64 0.058 and 0.093, 16 x 10 of 64 0.321 and 0.227; 100 of 192
+// 1.11 and 0.69, of 64 0.27 and 0.63; 10 of 2500 3.35 and 2.37, of 4000 5.3 and
+// 8.1; 8 x 10 of 800 1.25 and 0.95, 16 x 10 1.43 and 1.78.
+bool sweep_by_inverses(int count, const int64_t* n, const int64_t* b) {
+  double bytes = 0, links = 0, inv_flops = 0;
+  int64_t maxn = 0, maxq = 0;
+  for (int k = 0; k < count; ++k) bytes += 16.0 * n[k] * b[k] * b[k];
+  // a link: 64 rows and nothing to wait for but the step before; tiles that L2
+  // still holds; tiles from memory
+  const double warm = bytes < 50e6 ? 3.5e-6 : 7.8e-6;
   for (int k = 0; k < count; ++k) {
-    const double bb = (double)b[k] * b[k];
-    chain = std::max(chain, (double)n[k] * ((b[k] + 63) / 64) * 10e-6);
-    tile_bytes += 8.0 * (1.5 * n[k] * bb + (double)n[k] * a[k] * b[k]);
-    inv_flops += (double)n[k] * bb * b[k] / 3.0;
-    inv_bytes += 8.0 * (2.0 * n[k] * bb);
+    const int64_t q = (b[k] + 63) / 64;
+    links = std::max(links, (double)n[k] * q * (q == 1 ? 2.7e-6 : warm));
+    inv_flops += (double)n[k] * b[k] * b[k] * b[k] / 3.0;
     maxn = std::max(maxn, n[k]);
+    maxq = std::max(maxq, q);
   }
-  const double t_tile = std::max(chain, tile_bytes / 2e12);
-  const double t_inv = inv_flops / 20e12 + inv_bytes / 5e12 + maxn * 15e-6;
+  const double t_tile = 15e-6 + count * 18e-6 + std::max(links, 0.75 * bytes / 1.5e12);
+  const double t_inv = 10e-6 + count * 9e-6 + std::max(inv_flops / 36e12, maxq * 10e-6) + maxn * 7.5e-6 + bytes / 1.6e12;
   return t_inv < t_tile;
 }
 
@@ -722,7 +729,7 @@ int bta_pobtas_batched(bta_handle_t h, int count, const int64_t* n, const int64_
         (a[k] > 0 && (!Ab || !T || !Ab[k] || !T[k])) || b[k] > INT32_MAX / 2)
       return BTA_ERR_INVALID;
   }
-  if (sweep_by_inverses(count, n, b, a)) {
+  if (sweep_by_inverses(count, n, b)) {
     // block inverses of C steps at a time (about 1 GiB for all instances),
     // each chunk then swept by one persistent launch
     std::vector<int> ni(count), bi(count), ai(count), vlo(count, 0);
@@ -749,41 +756,44 @@ int bta_pobtas_batched(bta_handle_t h, int count, const int64_t* n, const int64_
       need += align_up(C * (size_t)b[k] * b[k] * 8);
     }
     need += align_up(nflags * sizeof(int));
-    int rc = ensure_ws(h, need);
-    if (rc) return rc;
-    cudaStream_t s = h->stream;
-    Carve cv{h->ws};
-    double* work = cv.take<double>(sweep_inv_work_total(count, ni.data(), bi.data(), ai.data()) + apart);
-    int* flags = cv.take<int>(nflags);
-    for (int k = 0; k < count; ++k) {
-      vbuf[k] = cv.take<double>(C * (size_t)b[k] * b[k]);
-      Vk[k] = vbuf[k];
-    }
-    if (trans == 1)
-      for (int k = 0; k < count; ++k)
-        if (a[k] > 0 && arrow_backward(T[k], rhs[k], ni[k], bi[k], ai[k], s)) return BTA_ERR_CUDA;
-    for (int64_t s0 = 0; s0 < maxn; s0 += C) {
-      const int64_t s1 = std::min(maxn, s0 + C);
-      std::vector<TrtriInst> tr;
+    const int rc = ensure_ws(h, need);
+    if (rc && rc != BTA_ERR_ALLOC) return rc;
+    if (!rc) {
+      cudaStream_t s = h->stream;
+      Carve cv{h->ws};
+      double* work = cv.take<double>(sweep_inv_work_total(count, ni.data(), bi.data(), ai.data()) + apart);
+      int* flags = cv.take<int>(nflags);
       for (int k = 0; k < count; ++k) {
-        const int64_t e = std::min(s1, n[k]), cnt = e - s0;
-        if (cnt <= 0) continue;
-        const int64_t lo = trans == 0 ? s0 : n[k] - e;
-        const size_t bb = (size_t)b[k] * b[k];
-        tr.push_back({D[k] + lo * bb, vbuf[k], (int)cnt, bi[k]});
-        vlo[k] = (int)lo;
+        vbuf[k] = cv.take<double>(C * (size_t)b[k] * b[k]);
+        Vk[k] = vbuf[k];
       }
-      if (block_trtri(tr.data(), (int)tr.size(), flags, h->ctl, s)) return BTA_ERR_CUDA;
-      if (sweep_inv_steps(count, ni.data(), bi.data(), ai.data(), Lk.data(), Abk.data(), Vk.data(), vlo.data(), rhs,
-                          trans, (int)s0, (int)s1, work, h->ctl, s))
-        return BTA_ERR_CUDA;
+      if (trans == 1)
+        for (int k = 0; k < count; ++k)
+          if (a[k] > 0 && arrow_backward(T[k], rhs[k], ni[k], bi[k], ai[k], s)) return BTA_ERR_CUDA;
+      for (int64_t s0 = 0; s0 < maxn; s0 += C) {
+        const int64_t s1 = std::min(maxn, s0 + C);
+        std::vector<TrtriInst> tr;
+        for (int k = 0; k < count; ++k) {
+          const int64_t e = std::min(s1, n[k]), cnt = e - s0;
+          if (cnt <= 0) continue;
+          const int64_t lo = trans == 0 ? s0 : n[k] - e;
+          const size_t bb = (size_t)b[k] * b[k];
+          tr.push_back({D[k] + lo * bb, vbuf[k], (int)cnt, bi[k]});
+          vlo[k] = (int)lo;
+        }
+        if (block_trtri(tr.data(), (int)tr.size(), flags, h->ctl, s)) return BTA_ERR_CUDA;
+        if (sweep_inv_steps(count, ni.data(), bi.data(), ai.data(), Lk.data(), Abk.data(), Vk.data(), vlo.data(), rhs,
+                            trans, (int)s0, (int)s1, work, h->ctl, s))
+          return BTA_ERR_CUDA;
+      }
+      if (trans == 0)
+        for (int k = 0; k < count; ++k) {
+          double* part = work + sweep_inv_work_total(count, ni.data(), bi.data(), ai.data());
+          if (a[k] > 0 && arrow_forward(Ab[k], T[k], rhs[k], ni[k], bi[k], ai[k], part, s)) return BTA_ERR_CUDA;
+        }
+      return cuda_rc(cudaGetLastError());
     }
-    if (trans == 0)
-      for (int k = 0; k < count; ++k) {
-        double* part = work + sweep_inv_work_total(count, ni.data(), bi.data(), ai.data());
-        if (a[k] > 0 && arrow_forward(Ab[k], T[k], rhs[k], ni[k], bi[k], ai[k], part, s)) return BTA_ERR_CUDA;
-      }
-    return cuda_rc(cudaGetLastError());
+    // no memory for a step's inverses: the tile sweep
   }
   size_t need = 4 * kAlign;
   for (int k = 0; k < count; ++k) {

@@ -101,3 +101,36 @@ def test_selected_inversion_in_parts(leave):
     assert rc == 0
     # the same digits and the same integer sums, launched in other groups
     assert _err(got, ref) <= 1e-12
+
+
+def test_sweeps_without_room_for_block_inverses():
+    """20 blocks of 1000 go through block inverses of 160 MB, or where those
+    cannot be had through the tile sweep, which needs 10 MB."""
+    import torch
+
+    from dalia_b200 import _lib
+
+    lib = _lib.load()
+    n, b, a = 20, 1000, 3
+    m = _bta(n, b, a, 3)
+    info = ctypes.c_int64(-1)
+    _lib.check(lib.bta_pobtaf_batched(_lib.handle().bind_stream(), *_args(n, b, a, m), ctypes.byref(info)), "pobtaf")
+    rhs = torch.ones(n * b + a, dtype=torch.float64, device="cuda")
+    xs, held = [], []
+    for leave in (None, 60):
+        h = _lib.Handle()
+        x = rhs.clone()
+        filler = None if leave is None else _fill(leave * MB)
+        rc = 0
+        for trans in (0, 1):
+            rc = rc or lib.bta_pobtas_batched(h.bind_stream(), *_args(n, b, a, m),
+                                              (ctypes.c_void_p * 1)(x.data_ptr()), trans)
+        rc = rc or lib.bta_get_status(h.bind_stream(), ctypes.byref(info))
+        held.append(h.workspace_bytes())
+        del filler, h
+        torch.cuda.empty_cache()
+        assert rc == 0
+        xs.append(x)
+    assert held[0] > 100 * MB > held[1]
+    # well-conditioned (eigenvalues near 4): rounding of b terms
+    assert _err([xs[1]], [xs[0]]) <= 1e-12
