@@ -591,7 +591,9 @@ class SpatioTemporalModel:
         info = ctypes.c_int64(0)
         rc = self.lib.bta_get_status(self.h.bind_stream(), ctypes.byref(info))
         if rc == _lib.BTA_ERR_NOT_SPD:
-            raise np.linalg.LinAlgError(f"precision matrix not positive definite (pivot {info.value})")
+            k, pivot = divmod(info.value, 1 << 40)  # matrix k of a launch counts its pivots from k 2^40
+            raise np.linalg.LinAlgError(f"precision matrix not positive definite (pivot {pivot}"
+                                        + (f" of the launch's matrix {k})" if k else ")"))
         _lib.check(rc, "status")
 
     # ------------------------------------------------------------ objective
