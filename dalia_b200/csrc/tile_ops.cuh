@@ -9,19 +9,6 @@ namespace tile {
 constexpr int T = TILE;
 constexpr int THREADS = 128;
 constexpr int SG = T + 4;  // stride of GEMM operand tiles (k-contiguous, conflict-free)
-constexpr int SC = T + 1;  // stride of Cholesky / inverse tiles
-constexpr int NPAIR = T * (T + 1) / 2;
-
-__device__ __forceinline__ int pair_off(int k) { return T * k - k * (k - 1) / 2; }
-
-// Lower-triangle (i, k), k <= i, pairs ordered by k: the trailing pairs of
-// Cholesky step j (k > j) are the suffix starting at pair_off(j + 1).
-__device__ __forceinline__ void build_pairs(uint16_t* pairs, int tid) {
-  for (int k = tid; k < T; k += THREADS) {
-    const int o = pair_off(k);
-    for (int i = k; i < T; ++i) pairs[o + i - k] = (uint16_t)((i << 8) | k);
-  }
-}
 
 // Load a rows x cols tile (leading dimension ld) into smem with stride S,
 // zero-filled to 64 x 64.  L2-only loads (data may come from other CTAs).
@@ -98,27 +85,6 @@ __device__ __forceinline__ void zero_acc(double (&acc)[2][4][4]) {
     for (int ni = 0; ni < 4; ++ni)
 #pragma unroll
       for (int e = 0; e < 4; ++e) acc[mi][ni][e] = 0.0;
-}
-
-// acc += X(64 x kw) * Y(64 x kw)^T; X, Y k-contiguous in smem (stride SG).
-// Warp (wm, wn) owns rows wm*32.., cols wn*32.. of the 64x64 product.
-__device__ __forceinline__ void mma_nt(const double* X, const double* Y, int kw, double (&acc)[2][4][4],
-                                       int wm, int wn, int g, int t) {
-  for (int kk = 0; kk < kw; kk += 4) {
-    double a[2][2], b[4];
-#pragma unroll
-    for (int mi = 0; mi < 2; ++mi) {
-      const int r = wm * 32 + mi * 16 + g;
-      a[mi][0] = X[r * SG + kk + t];
-      a[mi][1] = X[(r + 8) * SG + kk + t];
-    }
-#pragma unroll
-    for (int ni = 0; ni < 4; ++ni) b[ni] = Y[(wn * 32 + ni * 8 + g) * SG + kk + t];
-#pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
-#pragma unroll
-      for (int ni = 0; ni < 4; ++ni) dmma16x8x4(acc[mi][ni], a[mi][0], a[mi][1], b[ni]);
-  }
 }
 
 // acc[n] += rows 16 warp .. of X times columns 8 n .. of Y^T for a lower
