@@ -22,7 +22,7 @@
 // K-major shared-memory images the MMA reads) and gemm_i8_kernel, persistent
 // CTAs over 128 x 64 output tiles: one producer thread bulk-copies the digit
 // images of each 32-wide k-slab (A: 128 rows x OZ_S digits, B: 64 rows x OZ_S
-// digits, no multicast) into a 3-stage ring; one thread issues the products
+// digits, no multicast) into a ring of four stages; one thread issues the products
 // of the slab, one MMA per A digit p against the stacked B digits (N up to
 // 256: 10 MMAs for 28 digit pairs), each pair (p, q) landing in the TMEM
 // accumulator of d = p + q; eight epilogue warps (two per 32-lane quarter of
@@ -570,8 +570,8 @@ __global__ void __launch_bounds__(QTHREADS, 1) gemm_i8_kernel(const __grid_const
           const int nk = qseg_range<BN>(sg, tm * QBM, tn * BN, kt0);
           // A: the whole block; B: BN rows of each digit's image, from row
           // (tn BN) % 128 (a multiple of eight rows).  One piece for A and
-          // OZ_S for B: the single issuing thread bounded the kernel with
-          // OZ_S pieces for each (93 cycles a piece of a 1290-cycle slab).
+          // OZ_S for B: with OZ_S for each, at 93 cycles a piece, the single
+          // issuing thread took as long as a slab's products.
           const int8_t* pa = sg.A + ((size_t)kt0 * sg.RBa + tm) * A_BLOCK;
           const int8_t* pb = sg.B + ((size_t)kt0 * sg.RBb + (tn * BN) / QBM) * A_BLOCK + (tn * BN) % QBM * QBK;
           const size_t da = (size_t)sg.RBa * A_BLOCK, db = (size_t)sg.RBb * A_BLOCK;
@@ -786,9 +786,9 @@ inline size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 // problem the longest first, each to the CTA with the least work so far.
 // Tiles c, c + grid, ... leave CTAs with the same kind of tile when a
 // problem's k-ranges are triangular and its tiles per row divide the grid
-// evenly: L V and V^T V of 12 x 1500 took 934 us that way (506 + 241 apart),
-// with the list 739 us, and 584 us since A comes in one piece.  Cost of a tile: its k-slabs, plus three for
-// the accumulators' read-out that the next tile's products wait for.
+// evenly: L V and V^T V of 12 x 1500 took 1.26 times as long that way.  Cost of
+// a tile: its k-slabs, plus three for the accumulators' read-out that the next
+// tile's products wait for.
 template <int BN>
 std::vector<int> deal_tiles(const QBatch& b, int total, int grid) {
   std::vector<std::vector<int>> mine(grid);

@@ -369,8 +369,8 @@ __device__ __forceinline__ void lower_tile(int e, int& mi, int& ni) {
 // The loops of the write-back read a batch of rows from shared memory before
 // they store it (one row at a time: 4.0 k).  A step takes 28.5 k cycles
 // (potrf_inv 14.3, solve 4.5, update 3.7, write-back 2.8, loads 1.4, flag of X
-// 1.3) against 70 k for the first version; 10 blocks of 300: 1.82 -> 0.94 ms,
-// 20 blocks of 1500: 18.2 -> 9.5 ms.
+// 1.3): 50 steps of 10 blocks of 300 are 0.73 of 0.92 ms, 480 of 20 blocks of
+// 1500 7.0 of 9.5 ms.
 __device__ void run_chain(const PanelInst& I, int inst, double* bufA, double* bufL, int* abort_flag, int* s_ok) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, t = lane & 3;
@@ -701,8 +701,8 @@ __global__ void __launch_bounds__(THREADS, 3) panel_kernel(const __grid_constant
     // X(p, r) = (A(p, r) - acc) Linv_r^T: the inverse is fetched beside the
     // tile when it is there (else 1 k cycles a task are lost where the queue is
     // the bound), and after it otherwise, so that only the solve itself
-    // follows the inverse's release.  With the above: 10 blocks of 300 993 ->
-    // 944 us, 24 of 617 5.18 -> 5.08 ms, 20 of 1500 9.55 -> 9.46 ms.
+    // follows the inverse's release (5 % for 10 blocks of 300, 1 % for 20 of
+    // 1500, together with the first chain inputs' release by TASK_PREV).
     const bool early_linv = s_linv != 0;
     if (early_linv) load_async<SG>(bufL, I.Linv + (size_t)r * T * T, T, T, T, tid);
     frag_rsub(c.ptr, ld, c.rows, c.cols, acc, wm, wn, g, t);

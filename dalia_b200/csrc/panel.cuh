@@ -83,7 +83,9 @@ struct PanelBatch {
 // the diagonal), or accumulation followed by the TRSM with the inverse of the
 // column's diagonal tile.
 // TASK_TIP subtracts the panel's arrow rows from the tip: T -= X_a X_a^T.
-// TASK_PREV applies the previous block column's term to one tile (no waits).
+// TASK_PREV applies the previous block column's term to one tile: without
+// waits in a launch of one block column, in a whole-factorisation launch as
+// that column's tiles become final.
 enum : int { TASK_AGG_DIAG = 3, TASK_AGG_SUB = 4, TASK_AGG_TRSM = 5, TASK_TIP = 6, TASK_PREV = 7 };
 
 // Tile columns by which the previous-column tasks run ahead of the tiles'

@@ -186,8 +186,7 @@ __device__ __forceinline__ void potrf_inv_trailing(double* S, double* V, int war
 // In-place lower Cholesky of the 64x64 smem tile S and the inverse of its
 // factor in V (both stride SG), in 16-wide panels.  Rows and columns from w
 // to the end of their panel are treated as the identity, panels beyond are
-// left out (some 3.6 k cycles each: 20 blocks of 1500, whose last tile has 28
-// columns, 9.467 -> 9.440 ms, 24 of 617 with 41 5.08 -> 5.07 ms).  A
+// left out (some 3.6 k cycles each).  A
 // non-positive pivot j < w records base+j+1 in *info (atomicMin); the
 // factorisation continues.  On exit the lower triangles of S and V hold L and
 // L^-1 in the rows of those panels, their 16x16 diagonal blocks zeros above
