@@ -20,6 +20,7 @@ constexpr int TA_SLAB = T * TSK, TB_SLAB = TK * TSN;
 // shared memory: the ring (also the staging of a tile's sum, 64 x SG), then
 // the diagonal tile inverse (64 x SG)
 constexpr int TRTRI_RING = TST * (TA_SLAB + TB_SLAB) > T * SG ? TST * (TA_SLAB + TB_SLAB) : T * SG;
+constexpr int TRTRI_CTAS = 3;  // per SM, by registers and shared memory
 constexpr size_t TRTRI_SMEM = size_t(TRTRI_RING + T * SG) * sizeof(double);
 
 // One instance of a launch: n lower-triangular blocks of b x b at D, their
@@ -147,7 +148,7 @@ __device__ __forceinline__ bool trtri_stream(const double* Arow, int rows, const
 // The columns are not claimed by resident CTAs: the SMs take a long, a middle
 // and a short one each from the launch's order (claimed: 2 to 5 % slower).
 template <bool COL>
-__global__ void __launch_bounds__(THREADS, 3) block_trtri_kernel(const __grid_constant__ TrtriBatch B) {
+__global__ void __launch_bounds__(THREADS, TRTRI_CTAS) block_trtri_kernel(const __grid_constant__ TrtriBatch B) {
   extern __shared__ __align__(16) double sm[];
   double* As = sm;
   double* Ys = sm + TRTRI_RING;
@@ -363,14 +364,12 @@ size_t block_trtri_flags(int n, int b) {
 }
 
 int block_trtri(const TrtriInst* inst, int count, int* flags, int* abort_flag, cudaStream_t s) {
-  for (const void* f : {reinterpret_cast<const void*>(block_trtri_kernel<false>),
-                        reinterpret_cast<const void*>(block_trtri_kernel<true>)}) {
-    const int e = ensure_smem_attr(f, (int)TRTRI_SMEM);
+  if (count < 1) return cudaSuccess;
+  {
+    const int e = ensure_smem_attr(reinterpret_cast<const void*>(block_trtri_kernel<false>), (int)TRTRI_SMEM);
     if (e != cudaSuccess) return e;
   }
-  int occ = 0;
-  cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, block_trtri_kernel<false>, THREADS, TRTRI_SMEM);
-  if (e != cudaSuccess) return e;
+  cudaError_t e = cudaSuccess;
   for (int k0 = 0; k0 < count; k0 += TRTRI_MAXI) {
     TrtriBatch B;
     std::memset(&B, 0, sizeof(B));
@@ -400,7 +399,7 @@ int block_trtri(const TrtriInst* inst, int count, int* flags, int* abort_flag, c
     // (0.95) 14.6 and 14.0, 40 of 1500 (0.72) 1.88 and 1.85; 10 of 6000 (0.71)
     // 24.3 and 25.8, 14 of 4000 (0.66) 10.3 and 11.2, 20 of 1500 (0.36) 0.99 and
     // 1.52.  Blocks of one or two tiles gain nothing (1200 of 128: 0.124, 0.130).
-    const int slots = std::max(1, occ) * device_sm_count();
+    const int slots = TRTRI_CTAS * device_sm_count();
     const bool columns = nqmax > 2 && work >= COLUMN_WORK * (0.5 * nqmax * nqmax) * slots;
     if (total == 0) continue;
     if (total > INT32_MAX / 2) return cudaErrorInvalidValue;
@@ -418,6 +417,10 @@ int block_trtri(const TrtriInst* inst, int count, int* flags, int* abort_flag, c
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if (!columns) continue;
     B.total = (int)diag;  // as many columns
+    {
+      const int rc = ensure_smem_attr(reinterpret_cast<const void*>(block_trtri_kernel<true>), (int)TRTRI_SMEM);
+      if (rc != cudaSuccess) return rc;
+    }
     {
       bta::ProfScope _ps(bta::PROF_TRTRI, s);
       block_trtri_kernel<true><<<B.total, THREADS, TRTRI_SMEM, s>>>(B);
