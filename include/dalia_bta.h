@@ -273,7 +273,7 @@ int bta_panel_task_list_ex(int count, const int* b, const int* a, const int* fla
                            int* out, int cap, int* n_out);
 /* The queue of a whole FP64 factorisation in one launch (what
  * bta_pobtaf_batched runs when every arrow is at most 64 rows and its
- * workspace is at most 2 GiB; the environment variable
+ * workspace is at most 2 GiB and a quarter of the free memory; the variable
  * DALIA_B200_PANEL_PERSIST=1 / 0 forces it on / off): the
  * one-column queues of block columns 0, 1, ... one after the other, matrix k
  * having n[k] block columns (flags[k] bit 3: arrow tip); task field 0 is the
