@@ -480,8 +480,9 @@ int sweep_inv_steps(int count, const int* n, const int* b, const int* a, const d
     bmax = std::max(bmax, b[k]);
   }
   // candidates: a CTA per SM, or per two SMs (a quicker barrier, for small
-  // blocks); two on an SM do not fit (512 threads of 124 registers)
-  TuneLaunch tl("sweep", {count, trans, bsum, bmax, s1 - s0}, 2, s, 1);
+  // blocks); two on an SM do not fit (512 threads of 124 registers).  Each is
+  // tried twice: the first launch of a process also loads the kernel
+  TuneLaunch tl("sweep", {count, trans, bsum, bmax, s1 - s0}, 2, s);
   const int cand = tl.choice();
   PSweep P;
   std::memset(&P, 0, sizeof(P));

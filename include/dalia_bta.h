@@ -288,9 +288,8 @@ int bta_panel_task_list_all(int count, const int* b, const int* a, const int* fl
  * factorisation's kernel (queue order and lookahead, whether the chain CTAs
  * have their SMs to themselves) and of the persistent sweep (number of CTAs)
  * are tuned online:
- * the first launches of a new launch shape try every candidate (twice for
- * the factorisation's block columns, once for a sweep) on the real work,
- * timed by CUDA events, and the fastest is kept for that shape on that
+ * the first launches of a new launch shape try every candidate (twice) on
+ * the real work, timed by CUDA events, and the fastest is kept for that shape on that
  * device; the 8-bit-slice GEMM's output tile width (64, or 32 with two
  * tensor-memory accumulator sets) is chosen the same way per launch shape.
  * DALIA_B200_TUNE=0 turns it off; DALIA_B200_TUNE_CACHE=<file> reads earlier

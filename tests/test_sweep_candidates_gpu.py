@@ -20,10 +20,10 @@ def test_the_tuner_tries_two_sweep_launches(monkeypatch):
     L = torch.zeros(n - 1, b, b, dtype=torch.float64, device="cuda")
     x = torch.ones(n * b, dtype=torch.float64, device="cuda")
     one, ptr = ctypes.c_int64 * 1, ctypes.c_void_p * 1
-    for _ in range(4):
+    for _ in range(5):  # two candidates tried twice, then the decision
         _lib.check(lib.bta_pobtas_inv_batched(h.bind_stream(), 1, one(n), one(b), one(0), ptr(L.data_ptr()), None, None,
                                               ptr(V.data_ptr()), ptr(x.data_ptr()), 0), "sweep")
     torch.cuda.synchronize()
-    assert bool((x == 16.0).all())
+    assert bool((x == 32.0).all())
     line, = [ln for ln in _lib.tune_report() if ln.startswith("sweep|") and ":1,0,1237,1237,3 " in ln]
     assert len(line.split("ms=")[1].split(",")) == 2
