@@ -134,6 +134,19 @@ __device__ __forceinline__ bool trtri_stream(const double* Arow, int rows, const
   return ok;
 }
 
+// Zeros above the diagonal tile of tile column c (wc columns).
+__device__ __forceinline__ void zero_above(double* Oi, int b, int c, int wc, bool vec, int tid) {
+  for (int idx = 2 * tid; idx < c * T * T; idx += 2 * THREADS) {
+    double* z = Oi + (size_t)(idx >> 6) * b + c * T + (idx & 63);
+    if (vec && (idx & 63) + 1 < wc) {
+      *reinterpret_cast<double2*>(z) = make_double2(0.0, 0.0);
+    } else {
+      if ((idx & 63) < wc) z[0] = 0.0;
+      if ((idx & 63) + 1 < wc) z[1] = 0.0;
+    }
+  }
+}
+
 // Inverses of lower-triangular blocks, tile by tile:
 //   X(c, c) = Linv_cc,  X(p, c) = -Linv_pp sum_{k=c}^{p-1} L(p, k) X(k, c)   (p > c).
 // The sums are bound by the FP64 tensor pipe.
@@ -193,26 +206,17 @@ __global__ void __launch_bounds__(THREADS, TRTRI_CTAS) block_trtri_kernel(const 
     double* Oi = I.out + (size_t)i * b * b;
     int* gate = B.flags + I.flag0 + ((size_t)i * nq + c) * nq;
     const int wc = min(T, b - c * T);
+    // the task's (first) tile; its place is worked out here, where a task of one
+    // tile takes 1 us less than with it inside the loop below
+    const int p0 = COL ? c + 1 : c + s_task[3], rp0 = min(T, b - p0 * T);
+    double* o0 = Oi + (size_t)(p0 * T) * b + c * T;
     const bool vec = ((b & 1) == 0) &&
                      (((reinterpret_cast<uintptr_t>(Di) | reinterpret_cast<uintptr_t>(Oi)) & 15) == 0);
-    // above the diagonal tile
-    auto zeros = [&]() {
-      for (int idx = 2 * tid; idx < c * T * T; idx += 2 * THREADS) {
-        double* z = Oi + (size_t)(idx >> 6) * b + c * T + (idx & 63);
-        if (vec && (idx & 63) + 1 < wc) {
-          *reinterpret_cast<double2*>(z) = make_double2(0.0, 0.0);
-        } else {
-          if ((idx & 63) < wc) z[0] = 0.0;
-          if ((idx & 63) + 1 < wc) z[1] = 0.0;
-        }
-      }
-    };
-    if (s_task[3] == 0) {  // never with COL
-      double* o = Oi + (size_t)(c * T) * b + c * T;
+    if (p0 == c) {  // never with COL
       if (vec) load_async<SG>(As, Di + (size_t)(c * T) * b + c * T, b, wc, wc, tid);
       else load<SG>(As, Di + (size_t)(c * T) * b + c * T, b, wc, wc, tid);
       cp_async_commit();
-      if (B.zeros) zeros();
+      if (!COL && B.zeros) zero_above(Oi, b, c, wc, vec, tid);
       cp_async_wait<0>();
       __syncthreads();
       for (int r = wc + tid; r < T; r += THREADS) As[r * SG + r] = 1.0;
@@ -220,7 +224,7 @@ __global__ void __launch_bounds__(THREADS, TRTRI_CTAS) block_trtri_kernel(const 
       trinv(As, Ys, rd, tid);
       for (int idx = tid; idx < T * T; idx += THREADS) {
         const int r = idx >> 6, cc = idx & 63;
-        if (r < wc && cc < wc) o[(size_t)r * b + cc] = Ys[r * SG + cc];
+        if (r < wc && cc < wc) o0[(size_t)r * b + cc] = Ys[r * SG + cc];
       }
       __syncthreads();
       if (tid == 0) st_release(gate + c, 1);
@@ -229,14 +233,11 @@ __global__ void __launch_bounds__(THREADS, TRTRI_CTAS) block_trtri_kernel(const 
     // a tile, or the tiles of a column one after the other: those are read back
     // by this CTA alone (a barrier orders them)
     const bool own = COL && !B.zeros;  // COL: always
-    int p = COL ? c + 1 : c + s_task[3];
-    const int pend = COL ? nq : p + 1;
-    if (COL) {
-      zeros();
-    }
-    for (; p < pend; ++p) {
-      const int rp = min(T, b - p * T);
-      double* o = Oi + (size_t)(p * T) * b + c * T;
+    const int pend = COL ? nq : p0 + 1;
+    if (COL) zero_above(Oi, b, c, wc, vec, tid);
+    for (int p = p0; p < pend; ++p) {
+      const int rp = COL ? min(T, b - p * T) : rp0;
+      double* o = COL ? Oi + (size_t)(p * T) * b + c * T : o0;
       double acc[2][4][4];
       zero_acc(acc);
       const double* Arow = Di + (size_t)(p * T) * b;
